@@ -32,6 +32,8 @@ UNITS = [
     ("yee_f32.cu", []),
     ("leapfrog_f64.cu", ["--fmad=false"]),
     ("leapfrog_f32.cu", []),
+    ("resident_f64.cu", ["--fmad=false"]),
+    ("resident_f32.cu", []),
     ("sensors.cu", []),
     ("dft_tc.cu", []),
     ("voxel.cu", ["--fmad=false"]),
@@ -40,13 +42,14 @@ UNITS = [
     ("oblique.cu", ["--fmad=false"]),
     ("runtime.cpp", None),
     ("fused.cpp", None),
+    ("resident.cpp", None),
     ("tma.cpp", None),
     ("oblique_driver.cpp", None),
     ("batch.cpp", None),
     ("server.cpp", None),
 ]
 HEADERS = ["aefdtd_dev.hpp", "kernels.hpp", "sensors.cuh", "yee.cuh", "leapfrog.cuh", "sim.hpp", "mbar.cuh",
-           "interior_tma.cuh", "batch_persist.cuh", "pulse.cuh"]
+           "interior_tma.cuh", "batch_persist.cuh", "pulse.cuh", "resident.cuh"]
 
 
 def _stale(obj, deps):

@@ -189,6 +189,58 @@ template <typename T, typename Tid> struct PersistArgs {
     int withhold;                      // test hook: unit 0 never reports its progress
 };
 
+// ---- resident time steps (resident.cuh): a grid that stays on the SMs
+// A CTA's block: full x rows of rows [j0, j0 + by) and planes [k0, k0 + bz),
+// cut into runs of L planes per column (the kernels' L); thread
+// col + nx by run owns run `run` of column col = i + nx (j - j0).
+constexpr int kResRegions = 10;            // plane-sum planes (2) and DFT planes (kMaxGather)
+constexpr uint16_t kResNoRank = 0xffff;
+// The kernels that exist (resident_f32.cu, resident_f64.cu), by planes per run
+// and threads: short runs on 512 threads hide latency with warps, long runs on
+// 384 or 256 threads (up to 168 or 255 registers each) hold more cells per SM.
+struct ResKernel { int run, threads; };
+constexpr ResKernel kResKernels32[] = {{2, 512}, {4, 512}, {8, 384}, {12, 256}, {16, 256}, {20, 256}, {24, 256}};
+constexpr ResKernel kResKernels64[] = {{1, 512}, {2, 512}, {4, 384}, {6, 256}, {8, 256}, {10, 256}, {12, 256}};
+struct ResBlock {
+    int j0, by, k0, bz;
+    int nseg;                              // runs per column
+    unsigned feat_e, feat_h;               // features (kF* of yee.cuh) of the block's E and H updates
+    int nzp, npsi;                         // z-CPML planes in the block; psi slots per run (the launch's)
+    int self_y, self_z;                    // the block is its own neighbour along y / z
+    // shared-memory byte offsets (after fields and psi)
+    int o_halo, o_coef, o_z, o_inject, o_next, o_send, o_taps, o_sites, o_sum, o_rank, o_ids, o_disp, o_mats, o_poles;
+    int disp_off, disp_n;                  // dispersive cells
+    int tap_off, tap_n, site_off, site_n;  // sensor regions in the block, and their sites
+    // inbox offsets (in values): this block's own E and H halos (y face of
+    // 2 bz rows, then z face of 2 by rows, nx values each), and where its own
+    // faces go (the neighbours' inboxes; -1: its own neighbour)
+    int get_e, get_h, put_ey, put_ez, put_hy, put_hz;
+};
+struct ResDisp {
+    unsigned place;                        // shared-memory index (plane of the run x threads + thread) | material << 16
+    int psi;                               // element of psi: the cell in its material's box
+};
+// A block's part of a sensor region: sites [first, first + n) of the block's
+// (shared-memory index, place in a step's record), components stride apart in
+// the record; h: H too; region: its number (host).
+struct ResTaps { int first, n, stride, h, region; };
+template <typename T> struct ResArgs {
+    StepArgs<T, uint8_t> e, h;
+    const ResBlock *blocks;
+    const ResDisp *disp;
+    int npoles;                            // entries of e.crec, e.dchi
+    const ResTaps *taps;
+    const uint2 *sites;
+    unsigned long long *inbox;
+    T *raw;                                // [steps][rec]: sensor sites of every step of the launch
+    size_t rec;
+    int steps;
+    unsigned seq0;                         // half-steps numbered so far on this inbox
+    int *abort;
+    long long wait_cycles;                 // bound of each wait
+    int withhold;                          // test hook: block 0 skips its H updates
+};
+
 // ---- sensor-path launch arguments (kernels in sensors.cuh)
 
 struct PulseDev {
@@ -222,6 +274,17 @@ template <typename T> struct SensorStepArgs {
     GatherDesc g[kMaxGather];
     int part;                // 0: plane sums + E gathers (reads E only); 1: H gathers (reads H only)
     double *out;             // batch: plane-sum history [Nt][12]
+};
+
+// Sensor sites of `steps` resident steps: the interpolated samples of one DFT
+// plane from its recorded box of cells (sx x sy x sz sites, six components
+// `stride` apart), and the plane-sum planes of every step.
+template <typename T> struct ResGatherArgs {
+    const T *raw;            // record of the first step, at this region
+    size_t rec, stride;
+    int sx, sy, sz;
+    int type, span1, P;
+    T *S;                    // sample slot of the first step: [6][P] per step
 };
 
 // Single-wavelength field sensors (s_fieldmap.cpp): one launch per sensor

@@ -36,6 +36,11 @@ AEFDTD_DECL_FUSED(float, uint16_t)
 // (batch_persist.cuh), one cooperative launch of `grid` CTAs of 32 x ty
 // threads; persist_capacity: such CTAs resident on the current device at once
 template <typename T, typename Tid> int persist_capacity(int ty);
+// resident_f64.cu (--fmad=false) and resident_f32.cu: one cooperative launch
+// of `grid` CTAs that keep the whole grid on the SMs for A.steps steps; run:
+// planes per thread, one of kResKernels32 / kResKernels64
+cudaError_t launch_resident(const ResArgs<double> &A, int run, int grid, int smem, cudaStream_t s);
+cudaError_t launch_resident(const ResArgs<float> &A, int run, int grid, int smem, cudaStream_t s);
 #define AEFDTD_DECL_PERSIST(T, Tid)                                                                    \
     cudaError_t launch_persist(const PersistArgs<T, Tid> &p, int grid, int ty, cudaStream_t s);        \
     template <> int persist_capacity<T, Tid>(int ty);
@@ -54,6 +59,13 @@ AEFDTD_DECL_YEE(float, uint16_t)
 // one part (a.part) of a step's sensor work; returns the launches issued
 int launch_sensor_step(const SensorStepArgs<double> &a, cudaStream_t s);
 int launch_sensor_step(const SensorStepArgs<float> &a, cudaStream_t s);
+// resident steps: samples of one DFT plane for `steps` steps; plane-sum
+// partials of `steps` steps from the recorded planes (E components NxNy apart,
+// the reflection plane's three, then the transmission plane's)
+void launch_resident_gather(const ResGatherArgs<double> &a, int steps, cudaStream_t s);
+void launch_resident_gather(const ResGatherArgs<float> &a, int steps, cudaStream_t s);
+void launch_resident_planes(const SensorStepArgs<double> &a, const double *raw, size_t rec, int steps, cudaStream_t s);
+void launch_resident_planes(const SensorStepArgs<float> &a, const float *raw, size_t rec, int steps, cudaStream_t s);
 void launch_plane_reduce(const double *partial, int nbp, const StepScalars *sc, double *out, int steps,
                          cudaStream_t s);
 // completion sensor, FT mode: step a.q of every probe

@@ -140,6 +140,12 @@ void aefdtd_sim::construct(const aefdtd_grid_desc *d) {
     if (const char *tg = std::getenv("AEFDTD_TMA_STAGES")) tma_stages = atoi(tg) >= 6 ? 6 : 4;
     if (const char *tr = std::getenv("AEFDTD_TMA_RESERVE")) tma_reserve = std::clamp(atoi(tr), 0, 128);
     if (const char *tz = std::getenv("AEFDTD_TMA_PZ")) tma_pz = atoi(tz) != 0;
+    // resident time steps unless a knob pins the split kernels or their launches
+    for (const char *k : {"AEFDTD_KCHUNK", "AEFDTD_ZUNROLL", "AEFDTD_PREFETCH", "AEFDTD_HREV",
+                          "AEFDTD_PAIR", "AEFDTD_FUSED", "AEFDTD_TMA", "AEFDTD_TILE_Y", "AEFDTD_ALL_BOUNDARY",
+                          "AEFDTD_MERGE_PZ", "AEFDTD_MERGE_DISP", "AEFDTD_SERIAL_GROUPS"})
+        if (std::getenv(k)) use_resident = false;
+    if (const char *rs = std::getenv("AEFDTD_RESIDENT")) use_resident = atoi(rs) != 0;
     if (const char *ty = std::getenv("AEFDTD_TILE_Y")) {
         const int v = atoi(ty);
         tile_y = (v == 2 || v == 8) ? v : 4;
@@ -263,6 +269,7 @@ void aefdtd_sim::set_map(const uint32_t *m, size_t count) {
         AE_CUDA(cudaMemcpy(mat.p, v.data(), NP * 2, cudaMemcpyHostToDevice));
     }
     work_dirty = true;
+    res_dirty = true;
     map_set = true;
     tables_dirty = true;
 }
@@ -293,6 +300,7 @@ void aefdtd_sim::set_material(uint32_t idx, const aefdtd_material_desc *md) {
         h.C3 = 0;
         h.C4 = Dt / (e0 * h.ei);
         tables_dirty = true;
+        res_dirty = true;
         return;
     }
     std::vector<cplx> pa, pb;
@@ -343,6 +351,7 @@ void aefdtd_sim::set_material(uint32_t idx, const aefdtd_material_desc *md) {
     h.C4 = Dt / (e0 * e_eff);
     tables_dirty = true;
     work_dirty = true;
+    res_dirty = true;
     graphs_dirty = true;
 }
 
@@ -929,8 +938,11 @@ template <typename T, typename Tid>
 void aefdtd_sim::run_steps(int n) {
     // the staged kernels' tensor maps bake in the field and id arrays
     if (!work_dirty && (wsE.tma || wsH.tma) && !tma_maps_current()) work_dirty = true;
-    if (work_dirty) { build_work(); graphs_dirty = true; fwork_dirty = true; }
-    const bool fused = fused_eligible();
+    // a grid that fits the SMs' shared memory stays there (resident.cuh); the
+    // split path's work lists wait until they are needed
+    const bool resident = resident_ready();
+    if (work_dirty && !resident) { build_work(); graphs_dirty = true; fwork_dirty = true; }
+    const bool fused = !resident && fused_eligible();
     if (fused) {
         if (fwork_dirty) build_fused_work();
         ensure_other_set();
@@ -949,6 +961,10 @@ void aefdtd_sim::run_steps(int n) {
         psums_cap = cap;
         graphs_dirty = true;
         drop_graphs();
+    }
+    if (resident) {
+        run_resident<T>(n);
+        return;
     }
     if (obl && tstep + n > obl->cap) {
         obl_ensure(tstep + n);   // incident sums and R/T history (pointers the graphs bake in)
@@ -1526,6 +1542,7 @@ void aefdtd_sim::check_err() {
         AE_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), stream));
         // a staged launch that gave up may have left its unit counters set
         if (tma_ctr.p) AE_CUDA(cudaMemsetAsync(tma_ctr.p, 0, tma_ctr.n, stream));
+        if (res.abort.p) AE_CUDA(cudaMemsetAsync(res.abort.p, 0, res.abort.n, stream));
         fail(AEFDTD_TIMEOUT, "a bounded device wait ran out");
     }
 }
@@ -1555,6 +1572,7 @@ void aefdtd_sim::zero_state() {
     for (auto &b : psiH) if (b.p) AE_CUDA(cudaMemsetAsync(b.p, 0, b.n, stream));
     if (psi.p) AE_CUDA(cudaMemsetAsync(psi.p, 0, psi.n, stream));
     if (tma_ctr.p) AE_CUDA(cudaMemsetAsync(tma_ctr.p, 0, tma_ctr.n, stream));
+    if (res.abort.p) AE_CUDA(cudaMemsetAsync(res.abort.p, 0, res.abort.n, stream));
     if (obl) {
         for (int c = 0; c < 6; c++) {
             DBuf *b[3] = {&obl->Fi[c], &obl->psiEi[c], &obl->psiHi[c]};
@@ -1669,6 +1687,7 @@ aefdtd_status aefdtd_setup_normal(aefdtd_sim *s, const aefdtd_normal_desc *nd) {
         s->graphs_dirty = true;
         s->normal = true;
         s->work_dirty = true;
+        s->res_dirty = true;
     });
 }
 
@@ -1694,6 +1713,7 @@ aefdtd_status aefdtd_add_oscillator(aefdtd_sim *s, const aefdtd_source_desc *d, 
         o.step = s->tstep;
         s->oscs.push_back(o);
         s->work_dirty = true;
+        s->res_dirty = true;
         s->graphs_dirty = true;
         if (id) *id = (int32_t)s->oscs.size() - 1;
     });
@@ -1767,6 +1787,7 @@ aefdtd_status aefdtd_add_planar_sensor(aefdtd_sim *s, const aefdtd_sensor_desc *
         s->drain_sensors();
         s->sensors.push_back(p);
         s->graphs_dirty = true;
+        s->res_dirty = true;
         if (id) *id = (int32_t)s->sensors.size() - 1;
     });
 }
@@ -2395,6 +2416,11 @@ aefdtd_status aefdtd_test_hook(aefdtd_sim *s, int32_t what, int64_t value) {
             s->ps_wait_cycles = value;
         } else if (what == AEFDTD_TEST_PERSIST_WITHHOLD) {
             s->ps_withhold = value ? 1 : 0;
+        } else if (what == AEFDTD_TEST_RESIDENT_WAIT_CYCLES) {
+            if (value < 1) fail(AEFDTD_BAD_ARG, "wait bound must be at least 1 cycle");
+            s->res.wait_cycles = value;
+        } else if (what == AEFDTD_TEST_RESIDENT_WITHHOLD) {
+            s->res.withhold = value ? 1 : 0;
         } else {
             fail(AEFDTD_BAD_ARG, "unknown test hook");
         }

@@ -30,6 +30,22 @@ template <typename T> static void ccft_impl(const CcFtArgs<T> &a, cudaStream_t s
 void launch_completion_ft(const CcFtArgs<double> &a, cudaStream_t s) { ccft_impl(a, s); }
 void launch_completion_ft(const CcFtArgs<float> &a, cudaStream_t s) { ccft_impl(a, s); }
 int launch_fieldmap_step(const MapStepArgs<float> &a, cudaStream_t s) { return map_impl(a, s); }
+template <typename T> static void res_gather_impl(const ResGatherArgs<T> &a, int steps, cudaStream_t s) {
+    if (steps > 0 && a.P > 0)
+        resident_gather<<<dim3((a.P + kPlaneThreads - 1) / kPlaneThreads, steps), kPlaneThreads, 0, s>>>(a);
+}
+void launch_resident_gather(const ResGatherArgs<double> &a, int steps, cudaStream_t s) { res_gather_impl(a, steps, s); }
+void launch_resident_gather(const ResGatherArgs<float> &a, int steps, cudaStream_t s) { res_gather_impl(a, steps, s); }
+template <typename T>
+static void res_planes_impl(const SensorStepArgs<T> &a, const T *raw, size_t rec, int steps, cudaStream_t s) {
+    if (steps > 0 && a.nbp > 0) resident_planes<<<dim3(a.nbp, steps), kPlaneThreads, 0, s>>>(a, raw, rec);
+}
+void launch_resident_planes(const SensorStepArgs<double> &a, const double *raw, size_t rec, int steps, cudaStream_t s) {
+    res_planes_impl(a, raw, rec, steps, s);
+}
+void launch_resident_planes(const SensorStepArgs<float> &a, const float *raw, size_t rec, int steps, cudaStream_t s) {
+    res_planes_impl(a, raw, rec, steps, s);
+}
 void launch_plane_reduce(const double *partial, int nbp, const StepScalars *sc, double *out, int steps,
                          cudaStream_t s) {
     if (steps > 0) plane_sums_reduce<<<steps, 32, 0, s>>>(partial, nbp, sc, out);

@@ -22,9 +22,11 @@
 
 namespace aefdtd {
 
-// Block b of the plane-sum partials of step q (scalars a.sc[q]) into part[b*12 + c].
+// Block b of the plane-sum partials of step q (scalars a.sc[q]) into part[b*12 + c];
+// er, et: the reflection and the transmission plane's Ex, Ey, Ez, each Nx x Ny.
 template <typename T>
-__device__ __forceinline__ void plane_partial(const SensorStepArgs<T> &a, int b, int q, double *part) {
+__device__ __forceinline__ void plane_partial_at(const SensorStepArgs<T> &a, int b, int q, double *part,
+                                                 const T *const er[3], const T *const et[3]) {
     double acc[12];
 #pragma unroll
     for (int c = 0; c < 12; ++c) acc[c] = 0;
@@ -62,19 +64,18 @@ __device__ __forceinline__ void plane_partial(const SensorStepArgs<T> &a, int b,
             ty = pulse_eval(a.P, a.P.Ey0, x, y + Dy2, zt, tb);
             tz = pulse_eval(a.P, a.P.Ez0, x, y, zt + Dz2, tb);
         }
-        const long long ir = c + a.kr * a.NxNy, it = c + a.kt * a.NxNy;
         acc[0] = dadd(acc[0], dmul(bx, tap));
         acc[1] = dadd(acc[1], dmul(by, tap));
         acc[2] = dadd(acc[2], dmul(bz, tap));
-        acc[3] = dadd(acc[3], dmul(dsub((double)a.Ex[ir], bx), tap));
-        acc[4] = dadd(acc[4], dmul(dsub((double)a.Ey[ir], by), tap));
-        acc[5] = dadd(acc[5], dmul(dsub((double)a.Ez[ir], bz), tap));
+        acc[3] = dadd(acc[3], dmul(dsub((double)er[0][c], bx), tap));
+        acc[4] = dadd(acc[4], dmul(dsub((double)er[1][c], by), tap));
+        acc[5] = dadd(acc[5], dmul(dsub((double)er[2][c], bz), tap));
         acc[6] = dadd(acc[6], dmul(tx, tap));
         acc[7] = dadd(acc[7], dmul(ty, tap));
         acc[8] = dadd(acc[8], dmul(tz, tap));
-        acc[9] = dadd(acc[9], dmul((double)a.Ex[it], tap));
-        acc[10] = dadd(acc[10], dmul((double)a.Ey[it], tap));
-        acc[11] = dadd(acc[11], dmul((double)a.Ez[it], tap));
+        acc[9] = dadd(acc[9], dmul((double)et[0][c], tap));
+        acc[10] = dadd(acc[10], dmul((double)et[1][c], tap));
+        acc[11] = dadd(acc[11], dmul((double)et[2][c], tap));
     }
     __shared__ double red[12][kPlaneThreads];
 #pragma unroll
@@ -87,6 +88,12 @@ __device__ __forceinline__ void plane_partial(const SensorStepArgs<T> &a, int b,
         __syncthreads();
     }
     if (threadIdx.x < 12) part[b * 12 + threadIdx.x] = red[threadIdx.x][0];
+}
+template <typename T>
+__device__ __forceinline__ void plane_partial(const SensorStepArgs<T> &a, int b, int q, double *part) {
+    const long long ir = a.kr * a.NxNy, it = a.kt * a.NxNy;
+    const T *const er[3] = {a.Ex + ir, a.Ey + ir, a.Ez + ir}, *const et[3] = {a.Ex + it, a.Ey + it, a.Ez + it};
+    plane_partial_at(a, b, q, part, er, et);
 }
 
 // Fields interpolated to the node of cell (i, j, k): FDTD::local_E*/local_H*
@@ -246,6 +253,39 @@ __global__ void __launch_bounds__(kPlaneThreads) sensor_step(const __grid_consta
             gather_one(a, a.g[s], b);
             return;
         }
+}
+
+// Resident steps (resident.cuh), grid (blocks, steps). Plane sums: the same
+// blocks and order as plane_partial, over the planes recorded for every step.
+template <typename T>
+__global__ void __launch_bounds__(kPlaneThreads)
+resident_planes(const __grid_constant__ SensorStepArgs<T> a, const T *raw, size_t rec) {
+    const int q = blockIdx.y;
+    const T *p = raw + (size_t)q * rec;
+    const T *const er[3] = {p, p + a.NxNy, p + 2 * a.NxNy};
+    const T *const et[3] = {p + 3 * a.NxNy, p + 4 * a.NxNy, p + 5 * a.NxNy};
+    plane_partial_at(a, blockIdx.x, q, a.partial + (size_t)q * a.nbp * 12, er, et);
+}
+// The samples of one DFT plane: local_e and local_h over the recorded sites
+// (the wrapped neighbours are sites of their own).
+template <typename T>
+__global__ void __launch_bounds__(kPlaneThreads) resident_gather(const __grid_constant__ ResGatherArgs<T> a) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.P) return;
+    const T *r = a.raw + (size_t)blockIdx.y * a.rec;
+    const int u = p % a.span1, v = p / a.span1;
+    const int i = a.type <= 1 ? 0 : u, j = a.type <= 1 ? u : (a.type <= 3 ? 0 : v), k = a.type <= 3 ? v : 0;
+    auto F = [&](int c, int x, int y, int z) { return r[c * a.stride + x + (size_t)a.sx * (y + (size_t)a.sy * z)]; };
+    T f[6];
+    f[0] = (F(0, i, j, k) + F(0, i, j + 1, k) + F(0, i, j, k + 1) + F(0, i, j + 1, k + 1)) / T(4.0);
+    f[1] = (F(1, i, j, k) + F(1, i + 1, j, k) + F(1, i, j, k + 1) + F(1, i + 1, j, k + 1)) / T(4.0);
+    f[2] = (F(2, i, j, k) + F(2, i + 1, j, k) + F(2, i, j + 1, k) + F(2, i + 1, j + 1, k)) / T(4.0);
+    f[3] = (F(3, i, j, k) + F(3, i + 1, j, k)) / T(2.0);
+    f[4] = (F(4, i, j, k) + F(4, i, j + 1, k)) / T(2.0);
+    f[5] = (F(5, i, j, k) + F(5, i, j, k + 1)) / T(2.0);
+    T *S = a.S + (size_t)blockIdx.y * 6 * a.P;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) S[c * (long long)a.P + p] = f[c];
 }
 
 // Plane sums of L steps from their block partials, block q summing step q's

@@ -186,6 +186,31 @@ struct FieldMapHost {
     DBuf acc;
 };
 
+// Plan of the resident time steps (resident.cpp): blocks of the grid that stay
+// in shared memory, their inboxes, and the sensor sites recorded per step.
+struct ResRegion {
+    size_t base = 0, stride = 0;   // elements of a step's record
+    int x1 = 0, y1 = 0, z1 = 0, sx = 0, sy = 0, sz = 0;   // box of cells, wrapping
+    bool h = false;
+};
+struct ResidentPlan {
+    int grid = 0;                  // CTAs; 0: the grid does not run resident
+    int run = 0;                   // planes per thread
+    int smem = 0;
+    int cap = 0;                   // steps per launch
+    int nregions = 0;
+    size_t rec = 0;                // elements per step's record
+    ResRegion region[kResRegions];
+    unsigned seq = 0;              // half-steps numbered so far on the inboxes
+    long long wait_cycles = 1LL << 31;   // bound of each wait, and the test hook (aefdtd_test_hook)
+    int withhold = 0;
+    DBuf blocks, disp, taps, sites, raw, inbox, abort;
+    void release(size_t &t) {
+        for (DBuf *b : {&blocks, &disp, &taps, &sites, &raw, &inbox, &abort}) b->release(t);
+        grid = 0;
+    }
+};
+
 // Oblique driver state (FDTD_oblique_biphase_comp, oblique_biphase.cpp:29-330):
 // the imaginary grid's fields and CPML / dispersive state, the wideband Bloch
 // source (Bloch_Wideband, sc_bloch.cpp), phases and the R/T sum history.
@@ -380,6 +405,13 @@ struct aefdtd_sim {
     void swap_sets();
     template <typename T, typename Tid> void make_fused_args(FusedArgs<T, Tid> &A, const StepScalars *tbl, bool other);
     template <typename T, typename Tid> void enqueue_segment_fused(int L, StepScalars *tbl, bool record);
+    // resident time steps (resident.cuh): the whole grid in shared memory
+    bool use_resident = true;        // AEFDTD_RESIDENT
+    bool res_dirty = true;           // the map, a material, a source or a sensor changed
+    ResidentPlan res;
+    bool resident_ready();
+    void build_resident();
+    template <typename T> void run_resident(int n);
     // staged interior half-steps (interior_tma.cuh): curl-only 64 x 8 tiles
     // whose planes arrive through tensor copies. Not for batch members (their
     // merged lists take every interior item) or the oblique driver (whose
@@ -437,6 +469,7 @@ inline aefdtd_sim::~aefdtd_sim() {
     tables.release(t);
     for (auto &gx : graph_exec) if (gx.second) reap_graph(gx.second, device);
     items.release(t);
+    res.release(t);
     tma_units.release(t);
     tma_ctr.release(t);
     fm_tbl.release(t);

@@ -455,6 +455,14 @@ aefdtd_status aefdtd_probe_copy_bandwidth(int32_t device, size_t bytes, int32_t 
  * its next wait and the advance returns AEFDTD_TIMEOUT. */
 #define AEFDTD_TEST_PERSIST_WAIT_CYCLES 5
 #define AEFDTD_TEST_PERSIST_WITHHOLD 6
+/* The same for the resident time steps (a grid that stays in the SMs' registers
+ * and shared memory, taken when it fits): the bound of each wait for a
+ * neighbour block's values (default 2^31 cycles), and (value 1) a launch whose
+ * first block never updates H, so that its neighbours' waits run out; every
+ * CTA then leaves at its next barrier and the next synchronising call returns
+ * AEFDTD_TIMEOUT (reset the simulation before reuse). */
+#define AEFDTD_TEST_RESIDENT_WAIT_CYCLES 7
+#define AEFDTD_TEST_RESIDENT_WITHHOLD 8
 aefdtd_status aefdtd_test_hook(aefdtd_sim *sim, int32_t what, int64_t value);
 
 /* ---- batches: many simulations advanced together ----------------------
