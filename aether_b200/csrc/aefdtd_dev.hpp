@@ -198,17 +198,25 @@ constexpr uint16_t kResNoRank = 0xffff;
 // The kernels that exist (resident_f32.cu, resident_f64.cu), by planes per run
 // and threads: short runs on 512 threads hide latency with warps, long runs on
 // 384 or 256 threads (up to 168 or 255 registers each) hold more cells per SM.
-struct ResKernel { int run, threads; };
-constexpr ResKernel kResKernels32[] = {{2, 512}, {4, 512}, {8, 384}, {12, 256}, {16, 256}, {20, 256}, {24, 256}};
-constexpr ResKernel kResKernels64[] = {{1, 512}, {2, 512}, {4, 384}, {6, 256}, {8, 256}, {10, 256}, {12, 256}};
+// Tight ones share one exchange array between E and H.
+struct ResKernel { int run, threads; bool tight; };
+constexpr ResKernel kResKernels32[] = {{2, 512, false}, {4, 512, false}, {8, 384, false}, {12, 256, false}, {16, 256, false},
+                                       {20, 256, false}, {24, 256, false}, {25, 256, true}, {28, 256, true}};
+constexpr ResKernel kResKernels64[] = {{1, 512, false}, {2, 512, false}, {4, 384, false}, {6, 256, false}, {8, 256, false},
+                                       {10, 256, false}, {12, 256, false}, {13, 256, true}, {15, 256, true}};
+// Dispersive cells: poles per trip, and the cells a thread of a long run has in
+// flight through shared memory (res_ante_staged; 18 KB each in FP32, 36 in FP64).
+constexpr int kResPoles = 3;
+constexpr int res_stage(int bytes) { return bytes == 8 ? 1 : 2; }
+constexpr bool res_staged(int run, int bytes) { return run * bytes > 64; }
 struct ResBlock {
     int j0, by, k0, bz;
     int nseg;                              // runs per column
     unsigned feat_e, feat_h;               // features (kF* of yee.cuh) of the block's E and H updates
-    int nzp, npsi;                         // z-CPML planes in the block; psi slots per run (the launch's)
+    int nzp, npsi;                         // z-CPML planes in the block; psi slots per run
     int self_y, self_z;                    // the block is its own neighbour along y / z
     // shared-memory byte offsets (after fields and psi)
-    int o_halo, o_coef, o_z, o_inject, o_next, o_send, o_taps, o_sites, o_sum, o_rank, o_ids, o_disp, o_mats, o_poles;
+    int o_halo, o_coef, o_z, o_inject, o_next, o_taps, o_sites, o_sum, o_rank, o_ids, o_disp, o_poles, o_stage;
     int disp_off, disp_n;                  // dispersive cells
     int tap_off, tap_n, site_off, site_n;  // sensor regions in the block, and their sites
     // inbox offsets (in values): this block's own E and H halos (y face of

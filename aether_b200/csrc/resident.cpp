@@ -55,13 +55,22 @@ bool aefdtd_sim::resident_ready() {
 //
 // Cost of a step, in SM cycles of the slowest block (measured on cells of 12 to
 // 64 rows): per half-step 300, and per plane of its runs 40 (sending the
-// face) and per warp 11.5 (FP32) or 20 (FP64), twice that with z CPML, 2.5
-// times with poles, eight times in the rolled update (x/y CPML, oscillators);
-// 1700 per round of the threads over the dispersive cells, with 12 values per
-// pole read and written in L2 at about 50 bytes per cycle; 0.2 per halo value;
-// and 2600 for the two round trips of the inbox. Rows and planes are cut to
-// equal weights; pole state is concentrated in few rows and planes, so cuts
-// with its weight raised are tried too.
+// face) and per warp 11.5 (FP32), 20 or, past 13 planes, 30 (FP64), twice that
+// with z CPML, 2.5 times with poles, eight times in the rolled update (x/y
+// CPML, oscillators); per round of the threads over the dispersive cells 1700,
+// or 3500 in the long FP64 runs, in the short runs with 12 values per pole read
+// and written in L2 besides; the halo values past those that the threads read
+// in one round trip 0.75 (FP32) or 1.5 (FP64) each; and 2600 for the two round
+// trips of the inbox. Rows and planes are cut to equal weights; pole state is
+// concentrated in few rows and planes, so cuts with its weight raised are tried
+// too, and nearly equal cuts for the grids that fit no other.
+//
+// Where the line to the split half-steps lies: past kSlowest cycles the pole
+// state of a few blocks keeps all others waiting, which the split kernels
+// spread over the device. 60 x 60 x 200 FP32 with a disk of radius 18 (estimate
+// 24000): 13.1 against 16.8 us per step; with a sphere of radius 20 (34000)
+// 20.2 against 20.6; 48 x 48 x 200 FP64, disk of radius 12 (33000) 16.7 against
+// 20.1.
 void aefdtd_sim::build_resident() {
     res_dirty = false;
     res.grid = 0;
@@ -187,18 +196,27 @@ void aefdtd_sim::build_resident() {
         x.feat_e = kernel_feat(fe);
         x.feat_h = kernel_feat(f);
     };
-    // shared memory: fields, z psi, halo (and the reads of runs cut short past
-    // it), coefficients, z tables, injection values, thread records, sensor sites,
+    // psi slots of a block's runs: the planes from a run's first z-CPML plane to its last
+    auto slots = [&](const ResBlock &x, int run) {
+        int n = 0;
+        for (int r = 0; pz && r < x.nseg; r++) {
+            const int k = x.k0 + r * run, e = std::min(k + run, x.k0 + x.bz);
+            const bool low = k < pml[4], high = e > Nz - pml[5];
+            if (low || high) n = std::max(n, (high ? e : std::min(e, pml[4])) - (low ? k : std::max(k, Nz - pml[5])));
+        }
+        return n;
+    };
+    // shared memory: fields, z psi, halo (runs cut short read on behind it),
+    // coefficients, z tables, injection values, thread records, sensor sites,
     // ids, pole sums and their ranks
-    auto layout = [&](ResBlock &x, const ResKernel &K, int npsi) -> size_t {
+    auto layout = [&](ResBlock &x, const ResKernel &K) -> size_t {
         const int run = K.run;
-        x.npsi = npsi;
-        size_t o = size_t(6 * run + 4 * npsi) * K.threads * es;
+        x.npsi = slots(x, run);
+        size_t o = size_t((K.tight ? 3 : 6) * run + 4 * x.npsi) * K.threads * es;
         x.o_halo = (int)o;
-        o += up16((2 * size_t(Nx) * (x.by + x.bz) + std::max(run * Nx, K.threads)) * es);
+        o += up16(2 * size_t(Nx) * (x.by + x.bz) * es);
+        const size_t past = o + std::max(run * Nx, K.threads) * es;
         x.o_next = (int)o;
-        o += size_t(2) * K.threads * 16;
-        x.o_send = (int)o;
         o += size_t(2) * K.threads * 8;
         x.o_taps = (int)o;
         o += up16(size_t(kResRegions) * sizeof(ResTaps));
@@ -211,35 +229,39 @@ void aefdtd_sim::build_resident() {
         x.o_inject = (int)o;
         o += normal ? size_t(seg_len) * 4 * es : 0;
         x.o_ids = (int)o;
-        o += up16(size_t(run) * K.threads);
+        o += size_t((run + 3) / 4) * 4 * K.threads;
         x.o_sum = (int)o;
         o += up16(size_t(x.disp_n) * 3 * es);
         x.o_rank = (int)o;
         o += x.disp_n ? up16(size_t(run) * K.threads * 2) : 0;
         x.o_disp = (int)o;
-        o += up16(size_t(x.disp_n) * sizeof(ResDisp));
-        x.o_mats = (int)o;
-        o += x.disp_n ? up16(size_t(Nmat) * 12) : 0;
+        o += size_t(x.disp_n) * 16;
         x.o_poles = (int)o;
         o += x.disp_n ? size_t(poles) * 4 * es : 0;
-        return o;
+        x.o_stage = (int)o;
+        o += x.disp_n && res_staged(run, (int)es) ? size_t(K.threads) * res_stage((int)es) * kResPoles * 6 * es : 0;
+        return std::max(o, past);
     };
     // cycles of a half-step of a block of rows x planes with features f, and of a whole step
     auto half = [&](int rows, int planes, int runs, int run, unsigned f) {
-        const double c = (fp64 ? 20 : 11.5) * (f == 0 ? 1.0 : f & kXY ? 8.0 : f & kDisp ? 2.5 : 2.0);
+        const double c = (fp64 ? run > 13 ? 30 : 20 : 11.5) * (f == 0 ? 1.0 : f & kXY ? 8.0 : f & kDisp ? 2.5 : 2.0);
         const double warps = (Nx * rows * runs + 31) / 32, n = std::min(run, planes);
         return 300 + n * std::max(warps * c, 60.0) + 40.0 * n;
     };
     auto cost = [&](const ResBlock &x, const ResKernel &K) {
-        const int rounds = (x.disp_n + K.threads - 1) / K.threads;
-        return half(x.by, x.bz, x.nseg, K.run, x.feat_e) + half(x.by, x.bz, x.nseg, K.run, x.feat_h) +
-               0.2 * 4 * Nx * (x.by + x.bz) + 1700.0 * rounds + pole_cost(x.j0, x.j0 + x.by, x.k0, x.k0 + x.bz);
+        const bool staged = res_staged(K.run, (int)es);
+        const double words = 2.0 * Nx * (x.by + x.bz);
+        const double ante = x.disp_n == 0 ? 0
+                            : staged ? (fp64 ? 3500.0 : 1700.0) * ((x.disp_n + K.threads - 1) / K.threads)
+                                     : 1700.0 * ((x.disp_n + K.threads - 1) / K.threads) + pole_cost(x.j0, x.j0 + x.by, x.k0, x.k0 + x.bz);
+        return (K.tight ? 200 : 0) + half(x.by, x.bz, x.nseg, K.run, x.feat_e) + half(x.by, x.bz, x.nseg, K.run, x.feat_h) +
+               2 * (0.1 * words + (fp64 ? 1.5 * std::max(0.0, words - 4 * K.threads) : 0.75 * std::max(0.0, words - 8 * K.threads))) + ante;
     };
-    double best = 0;
-    ResKernel kernel{0, 0};
-    int psi_slots = 1;
+    const double kSlowest = fp64 ? 36000 : 30000;
+    double best = kSlowest;
+    ResKernel kernel{0, 0, false};
     std::vector<int> cy, cz;
-    for (const auto &w : {std::array{1.0, 1.25}, {1.0, 1.8}, {0.0, 1.5}, {4.0, 1.5}}) {
+    for (const auto &w : {std::array{1.0, 1.25}, {1.0, 1.8}, {1.0, 1.1}, {0.0, 1.5}, {4.0, 1.5}}) {
         if (w[0] != 1.0 && sum_p.back() == 0) continue;
         std::vector<double> wy, wz;
         weights(wy, wz, w[0], w[1]);
@@ -262,24 +284,21 @@ void aefdtd_sim::build_resident() {
                     const int runs = (deep + K.run - 1) / K.run;
                     if (Nx * tall * runs > K.threads) continue;
                     const double waits = nb * ns > 1 ? 2600 : 600;
-                    if (!cy.empty() && waits + 2 * half(tall, deep, runs, K.run, 0) >= best) continue;
+                    if (waits + 2 * half(tall, deep, runs, K.run, 0) >= best) continue;
                     double worst = waits;
-                    int npsi = 1;
                     std::vector<ResBlock> x(size_t(nb) * ns);
                     bool better = true;
                     for (int s = 0; s < ns && better; s++)
                         for (int b = 0; b < nb && better; b++) {
                             ResBlock &y = x[size_t(s) * nb + b];
                             fill(y, yc[b], yc[b + 1], zc[s], zc[s + 1], K.run);
-                            if (y.nzp > 0) npsi = std::max(npsi, std::min(K.run, y.bz));
                             worst = std::max(worst, waits + cost(y, K));
-                            better = y.disp_n < kResNoRank && (cy.empty() || worst < best);
+                            better = y.disp_n < kResNoRank && worst < best && !(K.tight && ((y.feat_e | y.feat_h) & kXY));
                         }
-                    for (size_t m = 0; m < x.size() && better; m++) better = layout(x[m], K, npsi) <= limit;
+                    for (size_t m = 0; m < x.size() && better; m++) better = layout(x[m], K) <= limit;
                     if (!better) continue;
                     best = worst;
                     kernel = K;
-                    psi_slots = npsi;
                     cy = yc;
                     cz = zc;
                 }
@@ -298,7 +317,7 @@ void aefdtd_sim::build_resident() {
         for (int b = 0; b < nb; b++) {
             ResBlock &x = at(s, b);
             fill(x, cy[b], cy[b + 1], cz[s], cz[s + 1], run);
-            smem = std::max(smem, layout(x, kernel, psi_slots));
+            smem = std::max(smem, layout(x, kernel));
             x.disp_off = ndisp;
             ndisp += x.disp_n;
             x.self_y = nb == 1;

@@ -25,10 +25,10 @@
 // the y+1 and z+1 blocks (fdtd_core.cpp:363-969; both wrap). The thread that
 // owns a cell at such a face stores each value, together with the number of
 // the half-step, as one 64-bit word into the neighbour's inbox (FP64: two
-// words of 32 data bits each), and the one thread there that needs it reads
-// the word until it carries the number it waits for: data and flag arrive
-// together, so there is no fence and no second round trip, and threads inside
-// the block do not wait at all. One inbox slot per value is enough: a value
+// words of 32 data bits each), and the neighbour brings its inbox into
+// shared memory before its update, reading until every word carries the number
+// it waits for: data and flag arrive together, so there is no fence and no
+// second round trip. One inbox slot per value is enough: a value
 // is overwritten only by its owner's next update of that field, which needs
 // the neighbour's next value at the same place, which the neighbour computed
 // after it had read the slot. All CTAs are resident (cooperative launch) and
@@ -96,35 +96,36 @@ __device__ __forceinline__ Coef4<double> coef4(const MatCoef<double> *c) {
 }
 
 // Shared memory of a CTA, in values of T from the start: E [3][L][threads],
-// H [3][L][threads], z-CPML psi [E 0, E 1, H 0, H 1][npsi][threads].
+// H [3][L][threads] (Tight: in the same place, see resident_steps), z-CPML psi
+// [E 0, E 1, H 0, H 1][npsi][threads], a slot for each plane from a run's first
+// CPML plane to its last.
 extern __shared__ __align__(16) unsigned char res_sm[];
 template <typename T, int L, int NT> __device__ __forceinline__ T *res_e(int c) { return reinterpret_cast<T *>(res_sm) + c * L * NT; }
-template <typename T, int L, int NT> __device__ __forceinline__ T *res_h(int c) { return reinterpret_cast<T *>(res_sm) + (3 + c) * L * NT; }
-// psi q of the thread's first plane, its planes NT apart; only blocks with CPML
-// planes need one slot per plane (npsi of them), all others keep zeros
-template <typename T, int L, int NT> __device__ __forceinline__ T *res_pz(int npsi, int q) {
-    return reinterpret_cast<T *>(res_sm) + (6 * L + q * npsi) * NT + threadIdx.x;
+template <typename T, int L, int NT, bool Tight> __device__ __forceinline__ T *res_h(int c) {
+    return reinterpret_cast<T *>(res_sm) + ((Tight ? 0 : 3) + c) * L * NT;
+}
+// psi q of the thread's first slot, its slots NT apart
+template <typename T, int L, int NT, bool Tight> __device__ __forceinline__ T *res_pz(int npsi, int q) {
+    return reinterpret_cast<T *>(res_sm) + ((Tight ? 3 : 6) * L + q * npsi) * NT + threadIdx.x;
 }
 
 // The injection plane alone (kFMisc adds the oscillator boxes).
 constexpr unsigned kFInject = 16;
 
-// What a thread knows about its run of cells for the whole launch.
+// A thread's run of cells for the whole launch. Its geometry is in the thread's
+// records in shared memory (ResNext), read where it is used: kept in registers
+// across the steps it would push the fields of the longer runs out of them.
 template <typename T, int L> struct ResThread {
     T e0[L], e1[L], e2[L], h0[L], h1[L], h2[L];
-    int t, i, J, K, nk;                 // thread; column; first plane and number of planes
-    int xm, xp;                         // threads of the neighbouring columns along x
-    bool mixed;                         // more than one material in the run
-    Coef4<T> v;                         // the run's coefficients otherwise
-    T C4;
-    unsigned ids[(L + 3) / 4];          // material ids, a byte each
+    int K;                              // first plane
 };
 // z-CPML values of one of the block's planes for E and for H. Outside a side's
 // range b keeps psi (which is zero there) and c adds nothing, so the updates
-// need no branch.
+// need no branch; planes without a slot read zero.
 template <typename T> struct alignas(16) ResZ { T ik, b, c, pad; };
-template <typename T, int L> __device__ __forceinline__ int res_id(const ResThread<T, L> &s, int k) {
-    return (s.ids[k >> 2] >> (8 * (k & 3))) & 0xff;
+// Material id of a thread's run plane k: a word of shared memory per four planes.
+template <int NT> __device__ __forceinline__ int res_id(const ResBlock &B, int k) {
+    return (res_sm + B.o_ids)[((k >> 2) * NT + threadIdx.x) * 4 + (k & 3)];
 }
 
 // ---- one cell
@@ -133,7 +134,7 @@ template <typename T, int L> __device__ __forceinline__ int res_id(const ResThre
 // below; writes the new E to n.
 template <typename T, int L, int NT, unsigned F>
 __device__ __forceinline__ void res_cell_e(const StepArgs<T, uint8_t> &a, const ResBlock &B, const Coef4<T> v, int m, int i,
-                                           int J, int K, int k, int t, int q, const T e[3], const T h[3], T hxj, T hzj,
+                                           int J, int K, int k, int slot, int t, int q, const T e[3], const T h[3], T hxj, T hzj,
                                            T hyi, T hzi, T hxm, T hym, T n[3]) {
     T ikx = 1, iky = 1, ikz = 1;
     if constexpr ((F & kFPmlXY) != 0) { ikx = __ldg(a.ikx + i); iky = __ldg(a.iky + J); }
@@ -175,7 +176,7 @@ __device__ __forceinline__ void res_cell_e(const StepArgs<T, uint8_t> &a, const 
                 by = __ldg(a.by + J); cy = __ldg(a.cy + J); qy0 = a.psi_y0[oy]; qy1 = a.psi_y1[oy];
             }
         }
-        T *p0 = res_pz<T, L, NT>(B.npsi, 0) + k * NT, *p1 = res_pz<T, L, NT>(B.npsi, 1) + k * NT;
+        T *p0 = res_pz<T, L, NT, false>(B.npsi, 0) + slot * NT, *p1 = res_pz<T, L, NT, false>(B.npsi, 1) + slot * NT;
         if (ze) { bz = __ldg(a.bz + K); cz = __ldg(a.cz + K); qz0 = *p0; qz1 = *p1; }
         // Ex: y block, then z block
         if constexpr ((F & kFPmlXY) != 0) {
@@ -222,7 +223,7 @@ __device__ __forceinline__ void res_cell_e(const StepArgs<T, uint8_t> &a, const 
 // H of one cell: exj, ezj the row above, eyi, ezi the column after, exk, eyk
 // the plane above.
 template <typename T, int L, int NT, unsigned F>
-__device__ __forceinline__ void res_cell_h(const StepArgs<T, uint8_t> &a, const ResBlock &B, int i, int J, int K, int k, int t, int q, const T e[3],
+__device__ __forceinline__ void res_cell_h(const StepArgs<T, uint8_t> &a, const ResBlock &B, int i, int J, int K, int slot, int q, const T e[3],
                                            const T h[3], T exj, T ezj, T eyi, T ezi, T exk, T eyk, T n[3]) {
     T ax = a.dtdmx, ay = a.dtdmy, az = a.dtdmz;
     if constexpr ((F & kFPmlXY) != 0) { ax = a.dtdmx * __ldg(a.ikx + i); ay = a.dtdmy * __ldg(a.iky + J); }
@@ -250,7 +251,7 @@ __device__ __forceinline__ void res_cell_h(const StepArgs<T, uint8_t> &a, const 
                 by = __ldg(a.by + J); cy = __ldg(a.cy + J); qy0 = a.psi_y0[oy]; qy1 = a.psi_y1[oy];
             }
         }
-        T *p0 = res_pz<T, L, NT>(B.npsi, 2) + k * NT, *p1 = res_pz<T, L, NT>(B.npsi, 3) + k * NT;
+        T *p0 = res_pz<T, L, NT, false>(B.npsi, 2) + slot * NT, *p1 = res_pz<T, L, NT, false>(B.npsi, 3) + slot * NT;
         if (zh) { bz = __ldg(a.bz + K); cz = __ldg(a.cz + K); qz0 = *p0; qz1 = *p1; }
         // Hx: y block, then z block
         if constexpr ((F & kFPmlXY) != 0) {
@@ -286,56 +287,85 @@ __device__ __forceinline__ void res_cell_h(const StepArgs<T, uint8_t> &a, const 
 // ---- one run
 // Where a run finds the row next to it: component 0 at element p of shared
 // memory, the other at p + d, planes sj apart, in the block's own arrays or in
-// the halo; and the plane next to it: elements z and z + dz. Two records per
-// thread (for E, for H), computed once per launch.
-struct alignas(16) ResNext {
-    int p, sj_d, z, dz;   // sj_d: sj | d << 12
+// the halo; the plane next to it: elements z and z + dz; and the thread of the
+// column next to it. A run that reads a halo is also at the face whose values
+// the block sends there, so the same places give those in the neighbour's
+// inbox (p - halo along y, z - halo along z).
+template <typename T> struct ResRow {
+    const T *row, *plane;
+    int sj, dj, dz, x;
+    int nk, lo, np;       // the run's planes, its first z-CPML plane and the planes to its last
+    int face_y, face_z;   // places in the halo, -1 for none
 };
-template <typename T, int L, int NT, int HALF> __device__ __forceinline__ ResNext res_next(int nx, const ResBlock &B, int t) {
-    const int ncol = nx * B.by, last = B.nseg - 1, run = t / ncol;
+// The record: two words per half-step and thread, computed once per launch.
+// p: element | halo << 16 | x << 17; z: element | halo << 16 | nk << 17 | lo << 22 | np << 27.
+template <int L> struct ResPack {
+    static_assert(L < 32, "a run's planes are packed in five bits");
+    static constexpr unsigned kHalo = 1u << 16;   // above any element of 227 KB
+};
+template <typename T, int L, int NT, bool Tight, int HALF>
+__device__ __forceinline__ uint2 res_pack(const StepArgs<T, uint8_t> &a, const ResBlock &B, int t) {
+    const int nx = a.Nx, ncol = nx * B.by, last = B.nseg - 1, run = t / ncol;
     // threads past the last run read what the first column reads
     const bool live = run <= last;
     const int seg = live ? run : 0, col = live ? t - run * ncol : 0, j = col / nx, i = col - j * nx, kb = seg * L;
-    const int base = HALF ? 0 : 3 * L * NT, halo = B.o_halo / (int)sizeof(T), own = live ? t : 0;
-    ResNext r;
+    const int base = HALF || Tight ? 0 : 3 * L * NT, halo = B.o_halo / (int)sizeof(T), own = live ? t : 0;
+    unsigned p, z;
     const bool edge = HALF ? j == B.by - 1 : j == 0;
-    if (!edge || B.self_y) {
-        r.p = base + own + (HALF ? (edge ? -j * nx : nx) : (edge ? (B.by - 1) * nx : -nx));
-        r.sj_d = NT | (2 * L * NT) << 12;
-    } else {
-        r.p = halo + kb * nx + i;
-        r.sj_d = nx | (nx * B.bz) << 12;
-    }
+    if (!edge || B.self_y) p = base + own + (HALF ? (edge ? -j * nx : nx) : (edge ? (B.by - 1) * nx : -nx));
+    else p = (halo + kb * nx + i) | ResPack<L>::kHalo;
     const bool end = HALF ? seg == last : seg == 0;
     if (!end || B.self_z) {
         const int k = HALF ? 0 : end ? B.bz - last * L - 1 : L - 1;
-        r.z = base + k * NT + own + (HALF ? (end ? -last * ncol : ncol) : (end ? last * ncol : -ncol));
-        r.dz = L * NT;
+        z = base + k * NT + own + (HALF ? (end ? -last * ncol : ncol) : (end ? last * ncol : -ncol));
     } else {
-        r.z = halo + 2 * nx * B.bz + col;
-        r.dz = ncol;
+        z = (halo + 2 * nx * B.bz + col) | ResPack<L>::kHalo;
     }
-    return r;
+    const int x = !live ? t : HALF ? (i < nx - 1 ? t + 1 : t - (nx - 1)) : (i ? t - 1 : t + nx - 1);
+    // planes of the run in [0, pml_zm) and [Nz - pml_zp, Nz)
+    const int K = B.k0 + kb, nk = live ? min(L, B.bz - kb) : 0;
+    const int low = a.pz ? max(0, min(nk, a.pml_zm - K)) : 0, high = a.pz ? min(nk, max(0, a.Nz - a.pml_zp - K)) : nk;
+    const int lo = low > 0 ? 0 : high, np = high < nk ? nk - lo : low;
+    return make_uint2(p | x << 17, z | nk << 17 | lo << 22 | unsigned(np) << 27);
 }
 template <typename T> __device__ __forceinline__ const T *res_at(int element) { return reinterpret_cast<const T *>(res_sm) + element; }
-template <int HALF> __device__ __forceinline__ ResNext res_record(const ResBlock &B, int nt) {
-    return reinterpret_cast<const ResNext *>(res_sm + B.o_next)[HALF * nt + threadIdx.x];
+template <typename T, int L, int NT, int HALF> __device__ __forceinline__ ResRow<T> res_record(int nx, const ResBlock &B) {
+    const uint2 w = reinterpret_cast<const uint2 *>(res_sm + B.o_next)[HALF * NT + threadIdx.x];
+    const bool hp = (w.x & ResPack<L>::kHalo) != 0, hz = (w.y & ResPack<L>::kHalo) != 0;
+    ResRow<T> r;
+    const int p = w.x & 0xffff, z = w.y & 0xffff, halo = B.o_halo / (int)sizeof(T);
+    r.row = res_at<T>(p);
+    r.plane = res_at<T>(z);
+    r.sj = hp ? nx : NT;
+    r.dj = hp ? nx * B.bz : 2 * L * NT;
+    r.dz = hz ? nx * B.by : L * NT;
+    r.x = w.x >> 17;
+    r.nk = w.y >> 17 & 31;
+    r.lo = w.y >> 22 & 31;
+    r.np = w.y >> 27;
+    r.face_y = hp && r.nk > 0 ? p - halo : -1;
+    r.face_z = hz && r.nk > 0 ? z - halo : -1;
+    return r;
 }
 
 // The run in registers, fully unrolled: any of pole sums, z CPML and the
 // injection plane; Mixed: the run holds several materials. Shared-memory
 // reads of a few planes at a time are issued together, psi is stored after
-// each such group and the fields after the whole run, so that no read waits
-// behind a store it cannot be told apart from. Planes past nk compute values
+// each such group and the fields (res_publish) after the whole run, so that no
+// read waits behind a store it cannot be told apart from. Planes past nk compute values
 // that nobody reads.
-template <typename T, int L, int NT, unsigned F, bool Mixed>
+template <typename T, int L, int NT, bool Tight, unsigned F, bool Mixed>
 __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B, ResThread<T, L> &s, int q) {
-    constexpr int C = sizeof(T) == 8 ? 2 : 4;
-    const ResNext next = res_record<0>(B, NT);
-    const T *row = res_at<T>(next.p), *plane = res_at<T>(next.z);
-    const int sj = next.sj_d & 0xfff, dj = next.sj_d >> 12, npsi = B.npsi;
+    constexpr int C = (sizeof(T) == 8 ? 2 : 4) / (L * (int)sizeof(T) > 104 ? 2 : 1);
+    const ResRow<T> next = res_record<T, L, NT, 0>(A.e.Nx, B);
+    const T *row = next.row, *plane = next.plane;
+    const int sj = next.sj, dj = next.dj, nk = next.nk, lo = next.lo;
     const MatCoef<T> *coef = reinterpret_cast<const MatCoef<T> *>(res_sm + B.o_coef);
     const ResZ<T> *zt = reinterpret_cast<const ResZ<T> *>(res_sm + B.o_z) + (s.K - B.k0);
+    // the run's coefficients where it has one material
+    const MatCoef<T> *const one = coef + res_id<NT>(B, 0);
+    const Coef4<T> v1 = coef4(one);
+    const T C41 = one->C4;
     // the run's plane that takes the injection, and its conducting plane
     const int kin = A.e.kinj - s.K, kpec = A.e.pz ? -s.K : -1;
     T injA = 0, injB = 0;
@@ -344,11 +374,14 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
         injA = inj[0];
         injB = inj[1];
     }
+    T *pz0 = res_pz<T, L, NT, Tight>(B.npsi, 0) - lo * NT, *pz1 = pz0 + B.npsi * NT;
     T hxm = plane[0], hym = plane[next.dz];
+    constexpr bool kBatchSums = sizeof(T) == 4;   // FP64 has no registers for a group's pole sums
 #pragma unroll
     for (int k0 = 0; k0 < L; k0 += C) {
-        if (k0 > 0 && k0 >= s.nk) break;
-        T yx[C], yz[C], x1[C], x2[C], p0[C], p1[C];
+        if (k0 > 0 && k0 >= nk) break;
+        T yx[C], yz[C], x1[C], x2[C], p0[C], p1[C], d0[C], d1[C], d2[C], C3[C];
+        int rank[C];
         Coef4<T> v[C];
         ResZ<T> z[C];
 #pragma unroll
@@ -357,20 +390,39 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
             if (k >= L) continue;
             yx[u] = row[k * sj];
             yz[u] = row[dj + k * sj];
-            x1[u] = res_h<T, L, NT>(1)[k * NT + s.xm];
-            x2[u] = res_h<T, L, NT>(2)[k * NT + s.xm];
-            if constexpr (Mixed) v[u] = coef4(coef + res_id(s, k));
+            x1[u] = res_h<T, L, NT, Tight>(1)[k * NT + next.x];
+            x2[u] = res_h<T, L, NT, Tight>(2)[k * NT + next.x];
+            if constexpr (Mixed) v[u] = coef4(coef + res_id<NT>(B, k));
+            if constexpr ((F & kFDisp) != 0) rank[u] = reinterpret_cast<const uint16_t *>(res_sm + B.o_rank)[k * NT + threadIdx.x];
             if constexpr ((F & kFPmlZ) != 0) {
                 z[u] = zt[k];
-                p0[u] = res_pz<T, L, NT>(npsi, 0)[min(k, npsi - 1) * NT];
-                p1[u] = res_pz<T, L, NT>(npsi, 1)[min(k, npsi - 1) * NT];
+                const bool slot = unsigned(k - lo) < unsigned(next.np);
+                p0[u] = slot ? pz0[k * NT] : T(0);
+                p1[u] = slot ? pz1[k * NT] : T(0);
+            }
+        }
+        if constexpr ((F & kFDisp) != 0 && kBatchSums) {
+            bool some = false;
+#pragma unroll
+            for (int u = 0; u < C; ++u) some |= k0 + u < L && rank[u] != kResNoRank;
+            if (some) {
+                const T *sum = reinterpret_cast<const T *>(res_sm + B.o_sum);
+#pragma unroll
+                for (int u = 0; u < C; ++u) {
+                    if (k0 + u >= L) continue;
+                    const int r = rank[u] != kResNoRank ? 3 * rank[u] : 0;
+                    d0[u] = sum[r];
+                    d1[u] = sum[r + 1];
+                    d2[u] = sum[r + 2];
+                    C3[u] = coef[res_id<NT>(B, k0 + u)].C3;
+                }
             }
         }
 #pragma unroll
         for (int u = 0; u < C; ++u) {
             const int k = k0 + u;
             if (k >= L) continue;
-            const Coef4<T> c = Mixed ? v[u] : s.v;
+            const Coef4<T> c = Mixed ? v[u] : v1;
             const T hx = s.h0[k], hy = s.h1[k], hz = s.h2[k];
             const T dHz_y = hz - yz[u], dHy_z = hy - hym, dHx_z = hx - hxm, dHz_x = hz - x2[u], dHy_x = hy - x1[u], dHx_y = hx - yx[u];
             T ikz = 1;
@@ -378,18 +430,21 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
             T nex = (c.C1 * s.e0[k] + c.C2y * dHz_y) - (c.C2z * ikz) * dHy_z;
             T ney = (c.C1 * s.e1[k] + (c.C2z * ikz) * dHx_z) - c.C2x * dHz_x;
             T nez = (c.C1 * s.e2[k] + c.C2x * dHy_x) - c.C2y * dHx_y;
-            if constexpr ((F & kFDisp) != 0) {
-                const int rank = reinterpret_cast<const uint16_t *>(res_sm + B.o_rank)[k * NT + s.t];
-                if (rank != kResNoRank) {
-                    const T C3 = coef[res_id(s, k)].C3;
-                    const T *sum = reinterpret_cast<const T *>(res_sm + B.o_sum) + 3 * rank;
-                    nex += C3 * sum[0];
-                    ney += C3 * sum[1];
-                    nez += C3 * sum[2];
+            if constexpr ((F & kFDisp) != 0)
+                if (rank[u] != kResNoRank) {
+                    if constexpr (!kBatchSums) {
+                        const T *sum = reinterpret_cast<const T *>(res_sm + B.o_sum) + 3 * rank[u];
+                        d0[u] = sum[0];
+                        d1[u] = sum[1];
+                        d2[u] = sum[2];
+                        C3[u] = coef[res_id<NT>(B, k)].C3;
+                    }
+                    nex += C3[u] * d0[u];
+                    ney += C3[u] * d1[u];
+                    nez += C3[u] * d2[u];
                 }
-            }
             if constexpr ((F & kFPmlZ) != 0) {
-                const T C4 = Mixed ? coef[res_id(s, k)].C4 : s.C4;
+                const T C4 = Mixed ? coef[res_id<NT>(B, k)].C4 : C41;
                 p0[u] = cpml_rec(z[u].b, p0[u], z[u].c, dHy_z);
                 nex -= C4 * p0[u];
                 p1[u] = cpml_rec(z[u].b, p1[u], z[u].c, dHx_z);
@@ -408,25 +463,19 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
         if constexpr ((F & kFPmlZ) != 0) {
 #pragma unroll
             for (int u = 0; u < C; ++u)
-                if (k0 + u < L && k0 + u < min(s.nk, npsi)) {
-                    res_pz<T, L, NT>(npsi, 0)[(k0 + u) * NT] = p0[u];
-                    res_pz<T, L, NT>(npsi, 1)[(k0 + u) * NT] = p1[u];
+                if (k0 + u < L && unsigned(k0 + u - lo) < unsigned(next.np)) {
+                    pz0[(k0 + u) * NT] = p0[u];
+                    pz1[(k0 + u) * NT] = p1[u];
                 }
         }
     }
-#pragma unroll
-    for (int k = 0; k < L; ++k) {
-        res_e<T, L, NT>(0)[k * NT + s.t] = s.e0[k];
-        res_e<T, L, NT>(1)[k * NT + s.t] = s.e1[k];
-        res_e<T, L, NT>(2)[k * NT + s.t] = s.e2[k];
-    }
 }
-template <typename T, int L, int NT, unsigned F>
+template <typename T, int L, int NT, bool Tight, unsigned F>
 __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B, ResThread<T, L> &s, int q) {
-    constexpr int C = sizeof(T) == 8 ? 2 : 4;
-    const ResNext next = res_record<1>(B, NT);
-    const T *row = res_at<T>(next.p), *plane = res_at<T>(next.z);
-    const int sj = next.sj_d & 0xfff, dj = next.sj_d >> 12, npsi = B.npsi;
+    constexpr int C = (sizeof(T) == 8 ? 2 : 4) / (L * (int)sizeof(T) > 104 ? 2 : 1);
+    const ResRow<T> next = res_record<T, L, NT, 1>(A.e.Nx, B);
+    const T *row = next.row, *plane = next.plane;
+    const int sj = next.sj, dj = next.dj, nk = next.nk, lo = next.lo;
     const ResZ<T> *zt = reinterpret_cast<const ResZ<T> *>(res_sm + B.o_z) + B.bz + L + (s.K - B.k0);
     const int kin = A.h.kinj - s.K, kpec = A.h.pz ? A.h.Nz - 1 - s.K : -1;
     T injA = 0, injB = 0;
@@ -436,10 +485,11 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
         injB = inj[3];
     }
     const T ax = A.h.dtdmx, ay = A.h.dtdmy, dtdmz = A.h.dtdmz, dtm = A.h.dtm;
+    T *pz0 = res_pz<T, L, NT, Tight>(B.npsi, 2) - lo * NT, *pz1 = pz0 + B.npsi * NT;
     const T zx = plane[0], zy = plane[next.dz];
 #pragma unroll
     for (int k0 = 0; k0 < L; k0 += C) {
-        if (k0 > 0 && k0 >= s.nk) break;
+        if (k0 > 0 && k0 >= nk) break;
         T yx[C], yz[C], x1[C], x2[C], p0[C], p1[C];
         ResZ<T> z[C];
 #pragma unroll
@@ -448,12 +498,13 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
             if (k >= L) continue;
             yx[u] = row[k * sj];
             yz[u] = row[dj + k * sj];
-            x1[u] = res_e<T, L, NT>(1)[k * NT + s.xp];
-            x2[u] = res_e<T, L, NT>(2)[k * NT + s.xp];
+            x1[u] = res_e<T, L, NT>(1)[k * NT + next.x];
+            x2[u] = res_e<T, L, NT>(2)[k * NT + next.x];
             if constexpr ((F & kFPmlZ) != 0) {
                 z[u] = zt[k];
-                p0[u] = res_pz<T, L, NT>(npsi, 2)[min(k, npsi - 1) * NT];
-                p1[u] = res_pz<T, L, NT>(npsi, 3)[min(k, npsi - 1) * NT];
+                const bool slot = unsigned(k - lo) < unsigned(next.np);
+                p0[u] = slot ? pz0[k * NT] : T(0);
+                p1[u] = slot ? pz1[k * NT] : T(0);
             }
         }
 #pragma unroll
@@ -461,7 +512,7 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
             const int k = k0 + u;
             if (k >= L) continue;
             const T ex = s.e0[k], ey = s.e1[k], ez = s.e2[k];
-            const bool end = k == L - 1 || k + 1 >= s.nk;
+            const bool end = k == L - 1 || k + 1 >= nk;
             const T exk = end ? zx : s.e0[k + (k < L - 1)], eyk = end ? zy : s.e1[k + (k < L - 1)];
             T az = dtdmz;
             if constexpr ((F & kFPmlZ) != 0) az = dtdmz * z[u].ik;
@@ -486,17 +537,22 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
         if constexpr ((F & kFPmlZ) != 0) {
 #pragma unroll
             for (int u = 0; u < C; ++u)
-                if (k0 + u < L && k0 + u < min(s.nk, npsi)) {
-                    res_pz<T, L, NT>(npsi, 2)[(k0 + u) * NT] = p0[u];
-                    res_pz<T, L, NT>(npsi, 3)[(k0 + u) * NT] = p1[u];
+                if (k0 + u < L && unsigned(k0 + u - lo) < unsigned(next.np)) {
+                    pz0[(k0 + u) * NT] = p0[u];
+                    pz1[(k0 + u) * NT] = p1[u];
                 }
         }
     }
+}
+
+// A run's field into its exchange array f.
+template <typename T, int L, int NT> __device__ __forceinline__ void res_publish(T *f, const T *c0, const T *c1, const T *c2) {
+    f += threadIdx.x;
 #pragma unroll
     for (int k = 0; k < L; ++k) {
-        res_h<T, L, NT>(0)[k * NT + s.t] = s.h0[k];
-        res_h<T, L, NT>(1)[k * NT + s.t] = s.h1[k];
-        res_h<T, L, NT>(2)[k * NT + s.t] = s.h2[k];
+        f[k * NT] = c0[k];
+        f[(L + k) * NT] = c1[k];
+        f[(2 * L + k) * NT] = c2[k];
     }
 }
 
@@ -505,20 +561,21 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
 // that the long body exists once and needs few registers.
 template <typename T, int L, int NT>
 __device__ __forceinline__ void res_run_e_all(const ResArgs<T> &A, const ResBlock &B, ResThread<T, L> &s, int q) {
-    const ResNext next = res_record<0>(B, NT);
-    const T *row = res_at<T>(next.p), *plane = res_at<T>(next.z);
-    const int sj = next.sj_d & 0xfff, dj = next.sj_d >> 12, npsi = B.npsi;
+    const ResRow<T> next = res_record<T, L, NT, 0>(A.e.Nx, B);
+    const T *row = next.row, *plane = next.plane;
+    const int sj = next.sj, dj = next.dj, t = threadIdx.x;
+    const int col = t - (s.K - B.k0) / L * (A.e.Nx * B.by), j = col / A.e.Nx, i = col - j * A.e.Nx, J = B.j0 + j;   // of a live run
     const MatCoef<T> *coef = reinterpret_cast<const MatCoef<T> *>(res_sm + B.o_coef);
     T hxm = plane[0], hym = plane[next.dz];
 #pragma unroll 1
-    for (int k = 0; k < s.nk; ++k) {
-        const int c = k * NT + s.t, x = k * NT + s.xm;
+    for (int k = 0; k < next.nk; ++k) {
+        const int c = k * NT + t, x = k * NT + next.x;
         const T e[3] = {res_e<T, L, NT>(0)[c], res_e<T, L, NT>(1)[c], res_e<T, L, NT>(2)[c]};
-        const T h[3] = {res_h<T, L, NT>(0)[c], res_h<T, L, NT>(1)[c], res_h<T, L, NT>(2)[c]};
-        const int m = reinterpret_cast<const uint8_t *>(res_sm + B.o_ids)[c];
+        const T h[3] = {res_h<T, L, NT, false>(0)[c], res_h<T, L, NT, false>(1)[c], res_h<T, L, NT, false>(2)[c]};
+        const int m = res_id<NT>(B, k);
         T n[3];
-        res_cell_e<T, L, NT, kFAll>(A.e, B, coef4(coef + m), m, s.i, s.J, s.K + k, k, s.t, q, e, h, row[k * sj], row[dj + k * sj],
-                                res_h<T, L, NT>(1)[x], res_h<T, L, NT>(2)[x], hxm, hym, n);
+        res_cell_e<T, L, NT, kFAll>(A.e, B, coef4(coef + m), m, i, J, s.K + k, k, k - next.lo, t, q, e, h, row[k * sj], row[dj + k * sj],
+                                res_h<T, L, NT, false>(1)[x], res_h<T, L, NT, false>(2)[x], hxm, hym, n);
         res_e<T, L, NT>(0)[c] = n[0];
         res_e<T, L, NT>(1)[c] = n[1];
         res_e<T, L, NT>(2)[c] = n[2];
@@ -527,73 +584,63 @@ __device__ __forceinline__ void res_run_e_all(const ResArgs<T> &A, const ResBloc
     }
 #pragma unroll
     for (int k = 0; k < L; ++k) {
-        const int c = k * NT + s.t;
+        const int c = k * NT + t;
         s.e0[k] = res_e<T, L, NT>(0)[c]; s.e1[k] = res_e<T, L, NT>(1)[c]; s.e2[k] = res_e<T, L, NT>(2)[c];
-        s.h0[k] = res_h<T, L, NT>(0)[c]; s.h1[k] = res_h<T, L, NT>(1)[c]; s.h2[k] = res_h<T, L, NT>(2)[c];
+        s.h0[k] = res_h<T, L, NT, false>(0)[c]; s.h1[k] = res_h<T, L, NT, false>(1)[c]; s.h2[k] = res_h<T, L, NT, false>(2)[c];
     }
 }
 template <typename T, int L, int NT>
 __device__ __forceinline__ void res_run_h_all(const ResArgs<T> &A, const ResBlock &B, ResThread<T, L> &s, int q) {
-    const ResNext next = res_record<1>(B, NT);
-    const T *row = res_at<T>(next.p), *plane = res_at<T>(next.z);
-    const int sj = next.sj_d & 0xfff, dj = next.sj_d >> 12, npsi = B.npsi;
+    const ResRow<T> next = res_record<T, L, NT, 1>(A.e.Nx, B);
+    const T *row = next.row, *plane = next.plane;
+    const int sj = next.sj, dj = next.dj, t = threadIdx.x;
+    const int col = t - (s.K - B.k0) / L * (A.e.Nx * B.by), j = col / A.e.Nx, i = col - j * A.e.Nx, J = B.j0 + j;   // of a live run
 #pragma unroll 1
-    for (int k = 0; k < s.nk; ++k) {
-        const int c = k * NT + s.t, x = k * NT + s.xp;
+    for (int k = 0; k < next.nk; ++k) {
+        const int c = k * NT + t, x = k * NT + next.x;
         const T e[3] = {res_e<T, L, NT>(0)[c], res_e<T, L, NT>(1)[c], res_e<T, L, NT>(2)[c]};
-        const T h[3] = {res_h<T, L, NT>(0)[c], res_h<T, L, NT>(1)[c], res_h<T, L, NT>(2)[c]};
-        const bool end = k + 1 >= s.nk;
+        const T h[3] = {res_h<T, L, NT, false>(0)[c], res_h<T, L, NT, false>(1)[c], res_h<T, L, NT, false>(2)[c]};
+        const bool end = k + 1 >= next.nk;
         const T exk = end ? plane[0] : res_e<T, L, NT>(0)[c + NT], eyk = end ? plane[next.dz] : res_e<T, L, NT>(1)[c + NT];
         T n[3];
-        res_cell_h<T, L, NT, kFPmlXY | kFPmlZ | kFMisc>(A.h, B, s.i, s.J, s.K + k, k, s.t, q, e, h, row[k * sj], row[dj + k * sj],
+        res_cell_h<T, L, NT, kFPmlXY | kFPmlZ | kFMisc>(A.h, B, i, J, s.K + k, k - next.lo, q, e, h, row[k * sj], row[dj + k * sj],
                                                     res_e<T, L, NT>(1)[x], res_e<T, L, NT>(2)[x], exk, eyk, n);
-        res_h<T, L, NT>(0)[c] = n[0];
-        res_h<T, L, NT>(1)[c] = n[1];
-        res_h<T, L, NT>(2)[c] = n[2];
+        res_h<T, L, NT, false>(0)[c] = n[0];
+        res_h<T, L, NT, false>(1)[c] = n[1];
+        res_h<T, L, NT, false>(2)[c] = n[2];
     }
 #pragma unroll
     for (int k = 0; k < L; ++k) {
-        const int c = k * NT + s.t;
+        const int c = k * NT + t;
         s.e0[k] = res_e<T, L, NT>(0)[c]; s.e1[k] = res_e<T, L, NT>(1)[c]; s.e2[k] = res_e<T, L, NT>(2)[c];
-        s.h0[k] = res_h<T, L, NT>(0)[c]; s.h1[k] = res_h<T, L, NT>(1)[c]; s.h2[k] = res_h<T, L, NT>(2)[c];
+        s.h0[k] = res_h<T, L, NT, false>(0)[c]; s.h1[k] = res_h<T, L, NT, false>(1)[c]; s.h2[k] = res_h<T, L, NT, false>(2)[c];
     }
 }
 
 // A run's face values into the neighbours' inboxes: E to the blocks below
-// (HALF 0), H to the blocks above (HALF 1); y, z: the run's places there (-1:
-// not at that face), in values.
-struct alignas(8) ResSend { int y, z; };
-template <int L, int NT, int HALF> __device__ __forceinline__ ResSend res_places(int nx, const ResBlock &B, int t) {
-    const int ncol = nx * B.by, run = t / ncol, col = t - run * ncol, j = col / nx;
-    ResSend r{-1, -1};
-    if (run >= B.nseg) return r;
-    const int put_y = HALF ? B.put_hy : B.put_ey, put_z = HALF ? B.put_hz : B.put_ez;
-    if (put_y >= 0 && j == (HALF ? B.by - 1 : 0)) r.y = put_y + run * L * nx + col - j * nx;
-    if (put_z >= 0 && run == (HALF ? B.nseg - 1 : 0)) r.z = put_z + col;
-    return r;
-}
+// (HALF 0), H to the blocks above (HALF 1).
 template <typename T, int L, int NT, int HALF>
 __device__ __forceinline__ void res_send(const ResArgs<T> &A, const ResBlock &B, const ResThread<T, L> &s, unsigned seq) {
-    const ResSend at = reinterpret_cast<const ResSend *>(res_sm + B.o_send)[HALF * NT + threadIdx.x];
     constexpr int kWords = sizeof(T) / 4;
     const int nx = A.e.Nx;
     const T *c0 = HALF ? s.h0 : s.e0, *c1 = HALF ? s.h1 : s.e1, *c2 = HALF ? s.h2 : s.e2;
-    if (at.z >= 0) {
+    const ResRow<T> at = res_record<T, L, NT, HALF>(nx, B);
+    if (at.face_z >= 0) {
         T x = c0[0], y = c1[0];
         if constexpr (HALF) {   // the run's last plane
 #pragma unroll
             for (int k = 1; k < L; ++k)
-                if (k < s.nk) { x = c0[k]; y = c1[k]; }
+                if (k < at.nk) { x = c0[k]; y = c1[k]; }
         }
-        unsigned long long *p = A.inbox + (size_t)at.z * kWords;
+        unsigned long long *p = A.inbox + (size_t)((HALF ? B.put_hz : B.put_ez) + at.face_z - 2 * nx * B.bz) * kWords;
         inbox_put(p, x, seq);
         inbox_put(p + nx * B.by * kWords, y, seq);
     }
-    if (at.y >= 0) {
-        unsigned long long *p = A.inbox + (size_t)at.y * kWords, *p2 = p + nx * B.bz * kWords;
+    if (at.face_y >= 0) {
+        unsigned long long *p = A.inbox + (size_t)((HALF ? B.put_hy : B.put_ey) + at.face_y) * kWords, *p2 = p + nx * B.bz * kWords;
 #pragma unroll
         for (int k = 0; k < L; ++k) {
-            if (k < s.nk) {
+            if (k < at.nk) {
                 inbox_put(p, c0[k], seq);
                 inbox_put(p2, c2[k], seq);
             }
@@ -673,63 +720,169 @@ __device__ __forceinline__ bool res_halo(const ResArgs<T> &A, const ResBlock &B,
 // Recursive-convolution "ante" update of the block's dispersive cells with
 // E^n (mats_RC.cpp:21-36), in the split kernels' order; the sums over poles
 // are kept for the E update. Cells, materials and pole coefficients are in
-// shared memory, so that a cell costs one round trip for its psi.
+// shared memory, so that a cell costs one round trip for its psi (and its
+// record one read: chains of table reads cost more than the psi). A thread
+// takes one component of a cell at a time, kResPoles poles of it per trip (with
+// whole cells the values in flight pushed the longer runs' fields out of the
+// registers).
 template <typename T> struct ResPole { Cplx<T> crec, dchi; };
-struct ResMat { int np, pole, box; };
-template <typename T, int L, int NT> __device__ __forceinline__ void res_ante(const ResArgs<T> &A, const ResBlock &B) {
-    const StepArgs<T, uint8_t> &a = A.e;
-    T *sum = reinterpret_cast<T *>(res_sm + B.o_sum);
-    const ResDisp *cells = reinterpret_cast<const ResDisp *>(res_sm + B.o_disp);
-    const ResMat *mats = reinterpret_cast<const ResMat *>(res_sm + B.o_mats);
-    const ResPole<T> *poles = reinterpret_cast<const ResPole<T> *>(res_sm + B.o_poles);
-    constexpr int kPoles = (NT == 512 ? 2 : 4) * 4 / (int)sizeof(T);   // in flight, beside the run's registers
-    for (int r = threadIdx.x; r < B.disp_n; r += NT) {
-        const ResDisp e = cells[r];
-        const ResMat m = mats[e.place >> 16];
-        const int c = e.place & 0xffff;
-        Cplx<T> *__restrict__ P = a.psi + e.psi;
-        const T ev[3] = {res_e<T, L, NT>(0)[c], res_e<T, L, NT>(1)[c], res_e<T, L, NT>(2)[c]};
-        T s[3] = {0, 0, 0};
-        for (int p0 = 0; p0 < m.np; p0 += kPoles) {
-            const int pn = min(kPoles, m.np - p0);
-            Cplx<T> v[kPoles][3];
-#pragma unroll
-            for (int p = 0; p < kPoles; ++p)
-                if (p < pn)
-#pragma unroll
-                    for (int dd = 0; dd < 3; ++dd) v[p][dd] = P[(3 * (p0 + p) + dd) * m.box];
-#pragma unroll
-            for (int p = 0; p < kPoles; ++p)
-                if (p < pn) {
-                    const ResPole<T> x = poles[m.pole + p0 + p];
-#pragma unroll
-                    for (int dd = 0; dd < 3; ++dd) {
-                        Cplx<T> w;
-                        if constexpr (Exact<T>::value) {
-                            w.re = (x.crec.re * v[p][dd].re - x.crec.im * v[p][dd].im) + x.dchi.re * ev[dd];
-                            w.im = (x.crec.re * v[p][dd].im + x.crec.im * v[p][dd].re) + x.dchi.im * ev[dd];
-                        } else {
-                            w.re = v[p][dd].re + ((x.crec.re * v[p][dd].re - x.crec.im * v[p][dd].im) + x.dchi.re * ev[dd]);
-                            w.im = v[p][dd].im + ((x.crec.re * v[p][dd].im + x.crec.im * v[p][dd].re) + x.dchi.im * ev[dd]);
-                        }
-                        P[(3 * (p0 + p) + dd) * m.box] = w;
-                        s[dd] = s[dd] + w.re;
-                    }
-                }
-        }
-        sum[3 * r] = s[0];
-        sum[3 * r + 1] = s[1];
-        sum[3 * r + 2] = s[2];
+struct alignas(16) ResCell { int psi, pole, box; unsigned short cell, np; };
+// Where the tables are, read once: shared memory is reread after every store.
+template <typename T> struct ResTables {
+    const ResCell *cells;
+    const ResPole<T> *poles;
+    T *sum;
+    Cplx<T> *psi;
+    int n;
+    __device__ ResTables(const ResArgs<T> &A, const ResBlock &B)
+        : cells(reinterpret_cast<const ResCell *>(res_sm + B.o_disp)), poles(reinterpret_cast<const ResPole<T> *>(res_sm + B.o_poles)),
+          sum(reinterpret_cast<T *>(res_sm + B.o_sum)), psi(A.e.psi), n(B.disp_n) {}
+};
+template <typename T> __device__ __forceinline__ Cplx<T> res_pole(const ResPole<T> &x, const Cplx<T> y, T e) {
+    Cplx<T> w;
+    if constexpr (Exact<T>::value) {
+        w.re = (x.crec.re * y.re - x.crec.im * y.im) + x.dchi.re * e;
+        w.im = (x.crec.re * y.im + x.crec.im * y.re) + x.dchi.im * e;
+    } else {
+        w.re = y.re + ((x.crec.re * y.re - x.crec.im * y.im) + x.dchi.re * e);
+        w.im = y.im + ((x.crec.re * y.im + x.crec.im * y.re) + x.dchi.im * e);
     }
+    return w;
+}
+// Item t: component t / n of dispersive cell t % n: its psi, E, poles, and where its sum goes.
+template <typename T> struct ResItem {
+    Cplx<T> *P;
+    T e;
+    int sum, pole, np, box;
+};
+template <typename T, int L, int NT> __device__ __forceinline__ ResItem<T> res_item(const ResTables<T> &X, int t) {
+    const int dd = (t >= X.n) + (t >= 2 * X.n), r = t - dd * X.n;
+    const ResCell c = X.cells[r];
+    return {X.psi + c.psi + dd * c.box, res_e<T, L, NT>(dd)[c.cell], 3 * r + dd, c.pole, c.np, 3 * c.box};
+}
+// Poles p0 to p0 + kResPoles of an item, their psi in v.
+template <typename T> __device__ __forceinline__ void res_poles(const ResPole<T> *poles, const ResItem<T> &x, int p0, const Cplx<T> *v, T &s) {
+#pragma unroll
+    for (int p = 0; p < kResPoles; ++p)
+        if (p0 + p < x.np) {
+            const Cplx<T> w = res_pole(poles[x.pole + p0 + p], v[p], x.e);
+            x.P[(p0 + p) * x.box] = w;
+            s = s + w.re;
+        }
+}
+template <typename T> __device__ __forceinline__ void res_poles_load(const ResItem<T> &x, int p0, Cplx<T> *v) {
+#pragma unroll
+    for (int p = 0; p < kResPoles; ++p)
+        if (p0 + p < x.np) v[p] = x.P[(p0 + p) * x.box];
+}
+// Asynchronous copy of one complex value to shared memory.
+__device__ __forceinline__ void res_fetch(Cplx<float> *to, const Cplx<float> *from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void res_fetch(Cplx<double> *to, const Cplx<double> *from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+// Short runs: U items in flight in registers.
+template <typename T, int L, int NT, int U> __device__ __forceinline__ void res_ante_direct(const ResArgs<T> &A, const ResBlock &B) {
+    const ResTables<T> X(A, B);
+    const int n = 3 * X.n;
+    for (int t0 = threadIdx.x; t0 < n; t0 += U * NT) {
+        ResItem<T> x[U];
+        Cplx<T> v[U][kResPoles];
+        T s[U];
+        int most = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            x[u].np = 0;
+            s[u] = 0;
+            if (t0 + u * NT < n) x[u] = res_item<T, L, NT>(X, t0 + u * NT);
+            most = max(most, x[u].np);
+        }
+        for (int p0 = 0; p0 < most; p0 += kResPoles) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) res_poles_load(x[u], p0, v[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) res_poles(X.poles, x[u], p0, v[u], s[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (t0 + u * NT < n) X.sum[x[u].sum] = s[u];
+    }
+}
+// Long runs leave no registers for psi in flight: the first poles of a thread's
+// next cells are copied ahead into shared memory, each thread its own.
+// Whole cells here, as with two warps per scheduler the instructions of a round
+// are what it costs: reading the tables once per cell instead of once per
+// component takes a third of them.
+template <typename T, int L, int NT> __device__ __forceinline__ void res_ante_staged(const ResArgs<T> &A, const ResBlock &B) {
+    const ResTables<T> X(A, B);
+    Cplx<T> *stage = reinterpret_cast<Cplx<T> *>(res_sm + B.o_stage) + threadIdx.x;
+    constexpr int D = res_stage(sizeof(T)), kVal = 3 * kResPoles;
+    const auto fetch = [&](int r) {
+        const int t = threadIdx.x + r * NT;
+        if (t < X.n) {
+            const ResCell c = X.cells[t];
+            const Cplx<T> *P = X.psi + c.psi;
+#pragma unroll
+            for (int p = 0; p < kResPoles; ++p)
+                if (p < c.np)
+#pragma unroll
+                    for (int dd = 0; dd < 3; ++dd) res_fetch(stage + (r % D * kVal + 3 * p + dd) * NT, P + (3 * p + dd) * c.box);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int r = 0; r < D; ++r) fetch(r);
+#pragma unroll 1
+    for (int r = 0; (int)threadIdx.x + r * NT < X.n; ++r) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+        const int t = threadIdx.x + r * NT;
+        const ResCell c = X.cells[t];
+        // FP64: a component at a time, for the registers
+        constexpr int W = sizeof(T) == 8 ? 1 : 3;
+#pragma unroll 1
+        for (int d0 = 0; d0 < 3; d0 += W) {
+            Cplx<T> *__restrict__ P = X.psi + c.psi + d0 * c.box;
+            const Cplx<T> *from = stage + (r % D * kVal + d0) * NT;
+            T e[W], s[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) { e[w] = res_e<T, L, NT>(d0 + w)[c.cell]; s[w] = 0; }
+            const auto pole = [&](int p, bool staged) {
+                const ResPole<T> x = X.poles[c.pole + p];
+                Cplx<T> v[W];
+#pragma unroll
+                for (int w = 0; w < W; ++w) v[w] = staged ? from[(3 * p + w) * NT] : P[(3 * p + w) * c.box];
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    const Cplx<T> y = res_pole(x, v[w], e[w]);
+                    P[(3 * p + w) * c.box] = y;
+                    s[w] = s[w] + y.re;
+                }
+            };
+#pragma unroll
+            for (int p = 0; p < kResPoles; ++p)
+                if (p < c.np) pole(p, true);
+#pragma unroll 1
+            for (int p = kResPoles; p < c.np; ++p) pole(p, false);
+#pragma unroll
+            for (int w = 0; w < W; ++w) X.sum[3 * t + d0 + w] = s[w];
+        }
+        fetch(r + D);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+template <typename T, int L, int NT> __device__ __forceinline__ void res_ante(const ResArgs<T> &A, const ResBlock &B) {
+    if constexpr (res_staged(L, sizeof(T))) res_ante_staged<T, L, NT>(A, B);
+    else res_ante_direct<T, L, NT, (NT > 256 ? 1 : 3)>(A, B);
 }
 
 // This step's values at the sites the sensors read (plane sums, DFT planes):
 // E (half 0) or H (half 1) from shared memory into the step's record, a site
 // per thread, region by region.
-template <typename T, int L, int NT>
+template <typename T, int L, int NT, bool Tight>
 __device__ __forceinline__ void res_taps(const ResArgs<T> &A, const ResBlock &B, int q, int half) {
     T *rec = A.raw + (size_t)q * A.rec;
-    const T *f = half ? res_h<T, L, NT>(0) : res_e<T, L, NT>(0);
+    const T *f = half ? res_h<T, L, NT, Tight>(0) : res_e<T, L, NT>(0);
     const ResTaps *region = reinterpret_cast<const ResTaps *>(res_sm + B.o_taps);
     const uint2 *site = reinterpret_cast<const uint2 *>(res_sm + B.o_sites);
     for (int r = 0; r < B.tap_n; ++r) {
@@ -749,20 +902,19 @@ __device__ __forceinline__ void res_taps(const ResArgs<T> &A, const ResBlock &B,
 }
 
 // z-CPML psi of a thread's run between global and shared memory.
-template <typename T, int L, int NT, bool Store>
-__device__ __forceinline__ void res_psi(const ResArgs<T> &A, const ResBlock &B, const ResThread<T, L> &s) {
+template <typename T, int L, int NT, bool Tight, bool Store>
+__device__ __forceinline__ void res_psi(const ResArgs<T> &A, const ResBlock &B, const ResThread<T, L> &s, int i, int J) {
+    const ResRow<T> at = res_record<T, L, NT, 0>(A.e.Nx, B);
     const StepArgs<T, uint8_t> &a = A.e;
     T *const g[4] = {A.e.psi_z0, A.e.psi_z1, A.h.psi_z0, A.h.psi_z1};
-    // a block with CPML planes has a slot for each of its run's planes
-    const int n = Store ? min(s.nk, B.npsi) : B.npsi;
 #pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        const int K = s.K + k;
-        const int zn = k >= s.nk ? -1 : K < a.pml_zm ? K : K >= a.Nz - a.pml_zp ? K - (a.Nz - a.pml_zp) + a.pml_zm : -1;
-        const long long o = s.i + (long long)s.J * a.Nx + zn * a.NxNy;
+    for (int n = 0; n < at.np; ++n) {
+        const int K = s.K + at.lo + n;
+        const int zn = K < a.pml_zm ? K : K >= a.Nz - a.pml_zp ? K - (a.Nz - a.pml_zp) + a.pml_zm : -1;
+        const long long o = i + (long long)J * a.Nx + zn * a.NxNy;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            T *p = res_pz<T, L, NT>(B.npsi, q) + k * NT;
+            T *p = res_pz<T, L, NT, Tight>(B.npsi, q) + n * NT;
             if constexpr (Store) {
                 if (zn >= 0) g[q][o] = *p;
             } else {
@@ -772,7 +924,12 @@ __device__ __forceinline__ void res_psi(const ResArgs<T> &A, const ResBlock &B, 
     }
 }
 
-template <typename T, int L, int NT>
+// Tight: E and H take turns in one exchange array. An update's neighbours' values
+// are read before its own result is published, with a barrier between, so the
+// field that a phase reads is always the one there. Half the shared memory per
+// cell for one barrier more per half-step; the blocks need the run updates
+// (res_run_e_all keeps both fields in shared memory).
+template <typename T, int L, int NT, bool Tight>
 __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ ResArgs<T> A) {
     __shared__ ResBlock B;
     const int tid = threadIdx.x;
@@ -782,30 +939,31 @@ __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ 
     const StepArgs<T, uint8_t> &a = A.e;
     const int nx = a.Nx;
     ResThread<T, L> s;
-    {
-        // threads past the last run shadow the first column with no planes of their own
+    uint2 *const rec = reinterpret_cast<uint2 *>(res_sm + B.o_next);
+    rec[tid] = res_pack<T, L, NT, Tight, 0>(a, B, tid);
+    rec[NT + tid] = res_pack<T, L, NT, Tight, 1>(a, B, tid);
+    // threads past the last run shadow the first column with no planes of their own
+    const auto column = [&](int &i, int &J, int &nk) {
         const int ncol = nx * B.by, run = tid / ncol, col = run < B.nseg ? tid - run * ncol : 0, j = col / nx;
-        const bool live = run < B.nseg;
-        s.t = tid;
-        s.i = col - j * nx;
-        s.J = B.j0 + j;
-        s.K = B.k0 + (live ? run * L : 0);
-        s.nk = !live ? 0 : min(L, B.bz - run * L);
-        s.xm = !live ? tid : s.i ? tid - 1 : tid + nx - 1;
-        s.xp = !live ? tid : s.i < nx - 1 ? tid + 1 : tid - (nx - 1);
-    }
+        i = col - j * nx;
+        J = B.j0 + j;
+        s.K = B.k0 + (run < B.nseg ? run * L : 0);
+        nk = run < B.nseg ? min(L, B.bz - run * L) : 0;
+    };
+    int i, J, nk;
+    column(i, J, nk);
     MatCoef<T> *coef = reinterpret_cast<MatCoef<T> *>(res_sm + B.o_coef);
-    uint8_t *ids = res_sm + B.o_ids;
+    unsigned *ids = reinterpret_cast<unsigned *>(res_sm + B.o_ids);
     for (int t = tid; t < a.nmat; t += NT) coef[t] = a.coef[t];
     if (B.disp_n > 0)
         for (int t = tid; t < L * NT; t += NT) reinterpret_cast<uint16_t *>(res_sm + B.o_rank)[t] = kResNoRank;
     // ---- load the run
-    const long long first = s.i + (long long)s.J * nx + s.K * a.NxNy;
-    s.mixed = false;
-    int id0 = 0;
+    const long long first = i + (long long)J * nx + s.K * a.NxNy;
+    bool mixed = false;   // more than one material in the run
+    unsigned id0 = 0, word = 0;
 #pragma unroll
     for (int k = 0; k < L; ++k) {
-        const bool live = k < s.nk;
+        const bool live = k < nk;
         const long long o = first + k * a.NxNy;
         s.e0[k] = live ? a.Ex[o] : T(0);
         s.e1[k] = live ? a.Ey[o] : T(0);
@@ -813,17 +971,15 @@ __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ 
         s.h0[k] = live ? a.Hx[o] : T(0);
         s.h1[k] = live ? a.Hy[o] : T(0);
         s.h2[k] = live ? a.Hz[o] : T(0);
-        const int m = live ? a.mat[s.i + (long long)a.mpitch * (s.J + (long long)a.Ny * (s.K + k))] : 0;
-        if ((k & 3) == 0) s.ids[k >> 2] = 0;
-        s.ids[k >> 2] |= (unsigned)m << (8 * (k & 3));
+        const unsigned m = live ? a.mat[i + (long long)a.mpitch * (J + (long long)a.Ny * (s.K + k))] : 0;
+        word = (k & 3) == 0 ? m : word | m << (8 * (k & 3));
+        if ((k & 3) == 3 || k == L - 1) ids[(k >> 2) * NT + tid] = word;
         if (k == 0) id0 = m;
-        s.mixed |= live && m != id0;
-        const int c = k * NT + tid;
-        ids[c] = (uint8_t)m;
-        res_e<T, L, NT>(0)[c] = s.e0[k]; res_e<T, L, NT>(1)[c] = s.e1[k]; res_e<T, L, NT>(2)[c] = s.e2[k];
-        res_h<T, L, NT>(0)[c] = s.h0[k]; res_h<T, L, NT>(1)[c] = s.h1[k]; res_h<T, L, NT>(2)[c] = s.h2[k];
+        mixed |= live && m != id0;
     }
-    res_psi<T, L, NT, false>(A, B, s);
+    res_publish<T, L, NT>(res_e<T, L, NT>(0), s.e0, s.e1, s.e2);
+    if constexpr (!Tight) res_publish<T, L, NT>(res_h<T, L, NT, false>(0), s.h0, s.h1, s.h2);
+    res_psi<T, L, NT, Tight, false>(A, B, s, i, J);
     {
         // the first E update's H halo, from the arrays
         const int jm = B.j0 == 0 ? a.Ny - 1 : B.j0 - 1, km = B.k0 == 0 ? a.Nz - 1 : B.k0 - 1;
@@ -842,8 +998,6 @@ __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ 
         }
     }
     __syncthreads();
-    s.v = coef4(coef + id0);
-    s.C4 = coef[id0].C4;
     // runs cut short read past the block's planes: those entries change nothing
     for (int t = tid; t < 2 * (B.bz + L); t += NT) {
         const bool h = t >= B.bz + L;
@@ -867,31 +1021,30 @@ __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ 
             inj[0] = (T)a.sc[q].inj_eA; inj[1] = (T)a.sc[q].inj_eB;
             inj[2] = (T)a.sc[q].inj_hA; inj[3] = (T)a.sc[q].inj_hB;
         }
-    {
-        ResNext *rec = reinterpret_cast<ResNext *>(res_sm + B.o_next);
-        rec[tid] = res_next<T, L, NT, 0>(nx, B, tid);
-        rec[NT + tid] = res_next<T, L, NT, 1>(nx, B, tid);
-        ResSend *places = reinterpret_cast<ResSend *>(res_sm + B.o_send);
-        places[tid] = res_places<L, NT, 0>(nx, B, tid);
-        places[NT + tid] = res_places<L, NT, 1>(nx, B, tid);
-    }
     for (int t = tid; t < B.tap_n; t += NT) reinterpret_cast<ResTaps *>(res_sm + B.o_taps)[t] = A.taps[B.tap_off + t];
     for (int t = tid; t < B.site_n; t += NT) reinterpret_cast<uint2 *>(res_sm + B.o_sites)[t] = A.sites[B.site_off + t];
-    const bool mixed = __any_sync(0xffffffffu, s.mixed);   // a warp takes one of the two forms
+    mixed = __any_sync(0xffffffffu, mixed);   // a warp takes one of the two forms
     if (B.disp_n > 0) {
         for (int t = tid; t < B.disp_n; t += NT) {
             const ResDisp e = A.disp[B.disp_off + t];
-            reinterpret_cast<ResDisp *>(res_sm + B.o_disp)[t] = e;
+            const DispInfo d = a.disp[e.place >> 16];
+            ResCell c;
+            c.psi = e.psi;
+            c.pole = d.pole_off;
+            c.box = (int)d.box;
+            c.cell = (unsigned short)e.place;
+            c.np = (unsigned short)d.np;
+            reinterpret_cast<ResCell *>(res_sm + B.o_disp)[t] = c;
             reinterpret_cast<uint16_t *>(res_sm + B.o_rank)[e.place & 0xffff] = (uint16_t)t;
-        }
-        for (int t = tid; t < a.nmat; t += NT) {
-            const DispInfo d = a.disp[t];
-            reinterpret_cast<ResMat *>(res_sm + B.o_mats)[t] = ResMat{d.np, d.pole_off, (int)d.box};
         }
         for (int t = tid; t < A.npoles; t += NT) reinterpret_cast<ResPole<T> *>(res_sm + B.o_poles)[t] = ResPole<T>{a.crec[t], a.dchi[t]};
     }
     __syncthreads();
     if (B.disp_n > 0) res_ante<T, L, NT>(A, B);
+    if constexpr (Tight) {
+        __syncthreads();
+        res_publish<T, L, NT>(res_h<T, L, NT, true>(0), s.h0, s.h1, s.h2);
+    }
     // half-step h of this launch carries number seq0 + h + 1
     bool ok = true;
 #pragma unroll 1
@@ -901,47 +1054,57 @@ __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ 
         if (!__syncthreads_and(ok)) return;
         switch (B.feat_e) {
             case 0:
-                if (mixed) res_run_e<T, L, NT, 0, true>(A, B, s, q);
-                else res_run_e<T, L, NT, 0, false>(A, B, s, q);
+                if (mixed) res_run_e<T, L, NT, Tight, 0, true>(A, B, s, q);
+                else res_run_e<T, L, NT, Tight, 0, false>(A, B, s, q);
                 break;
             case kFPmlZ | kFInject:
-                if (mixed) res_run_e<T, L, NT, kFPmlZ | kFInject, true>(A, B, s, q);
-                else res_run_e<T, L, NT, kFPmlZ | kFInject, false>(A, B, s, q);
+                if (mixed) res_run_e<T, L, NT, Tight, kFPmlZ | kFInject, true>(A, B, s, q);
+                else res_run_e<T, L, NT, Tight, kFPmlZ | kFInject, false>(A, B, s, q);
                 break;
-            case kFDisp | kFPmlZ | kFInject: res_run_e<T, L, NT, kFDisp | kFPmlZ | kFInject, true>(A, B, s, q); break;
-            default: res_run_e_all<T, L, NT>(A, B, s, q); break;
+            case kFDisp | kFPmlZ | kFInject: res_run_e<T, L, NT, Tight, kFDisp | kFPmlZ | kFInject, true>(A, B, s, q); break;
+            default:
+                if constexpr (!Tight) res_run_e_all<T, L, NT>(A, B, s, q);
+                break;
         }
+        if constexpr (Tight) __syncthreads();
+        res_publish<T, L, NT>(res_e<T, L, NT>(0), s.e0, s.e1, s.e2);
         res_send<T, L, NT, 0>(A, B, s, seq + 1);
         __syncthreads();
-        if (B.tap_n) res_taps<T, L, NT>(A, B, q, 0);
+        if (B.tap_n) res_taps<T, L, NT, Tight>(A, B, q, 0);
         // the next step's pole update, while the neighbours' E is on its way
         if (B.disp_n > 0 && q + 1 < A.steps) res_ante<T, L, NT>(A, B);
         ok = res_halo<T, NT, 1>(A, B, seq + 1);
         if (!__syncthreads_and(ok)) return;
         if (!(A.withhold && blockIdx.x == 0)) {
             switch (B.feat_h) {
-                case 0: res_run_h<T, L, NT, 0>(A, B, s, q); break;
-                case kFPmlZ | kFInject: res_run_h<T, L, NT, kFPmlZ | kFInject>(A, B, s, q); break;
-                default: res_run_h_all<T, L, NT>(A, B, s, q); break;
+                case 0: res_run_h<T, L, NT, Tight, 0>(A, B, s, q); break;
+                case kFPmlZ | kFInject: res_run_h<T, L, NT, Tight, kFPmlZ | kFInject>(A, B, s, q); break;
+                default:
+                    if constexpr (!Tight) res_run_h_all<T, L, NT>(A, B, s, q);
+                    break;
             }
+            if constexpr (Tight) __syncthreads();
+            res_publish<T, L, NT>(res_h<T, L, NT, Tight>(0), s.h0, s.h1, s.h2);
             res_send<T, L, NT, 1>(A, B, s, seq + 2);
         }
         __syncthreads();
-        if (B.tap_n) res_taps<T, L, NT>(A, B, q, 1);
+        if (B.tap_n) res_taps<T, L, NT, Tight>(A, B, q, 1);
     }
     // ---- store the run
+    column(i, J, nk);
+    const long long out = i + (long long)J * nx + s.K * a.NxNy;
 #pragma unroll
     for (int k = 0; k < L; ++k)
-        if (k < s.nk) {
-            const long long o = first + k * a.NxNy;
+        if (k < nk) {
+            const long long o = out + k * a.NxNy;
             a.Ex[o] = s.e0[k]; a.Ey[o] = s.e1[k]; a.Ez[o] = s.e2[k];
             a.Hx[o] = s.h0[k]; a.Hy[o] = s.h1[k]; a.Hz[o] = s.h2[k];
         }
-    if (B.nzp > 0) res_psi<T, L, NT, true>(A, B, s);
+    if (B.nzp > 0) res_psi<T, L, NT, Tight, true>(A, B, s, i, J);
 }
 
-template <typename T, int L, int NT> cudaError_t launch_resident_run(const ResArgs<T> &A, int grid, int smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(resident_steps<T, L, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+template <typename T, int L, int NT, bool Tight = false> cudaError_t launch_resident_run(const ResArgs<T> &A, int grid, int smem, cudaStream_t st) {
+    cudaError_t e = cudaFuncSetAttribute(resident_steps<T, L, NT, Tight>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -953,7 +1116,7 @@ template <typename T, int L, int NT> cudaError_t launch_resident_run(const ResAr
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, resident_steps<T, L, NT>, A);
+    return cudaLaunchKernelEx(&cfg, resident_steps<T, L, NT, Tight>, A);
 }
 
 }  // namespace aefdtd

@@ -11,6 +11,8 @@ cudaError_t launch_resident(const ResArgs<float> &A, int run, int grid, int smem
         case 16: return launch_resident_run<float, 16, 256>(A, grid, smem, s);
         case 20: return launch_resident_run<float, 20, 256>(A, grid, smem, s);
         case 24: return launch_resident_run<float, 24, 256>(A, grid, smem, s);
+        case 25: return launch_resident_run<float, 25, 256, true>(A, grid, smem, s);
+        case 28: return launch_resident_run<float, 28, 256, true>(A, grid, smem, s);
         default: return cudaErrorInvalidValue;
     }
 }

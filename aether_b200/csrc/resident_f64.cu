@@ -11,6 +11,8 @@ cudaError_t launch_resident(const ResArgs<double> &A, int run, int grid, int sme
         case 8: return launch_resident_run<double, 8, 256>(A, grid, smem, s);
         case 10: return launch_resident_run<double, 10, 256>(A, grid, smem, s);
         case 12: return launch_resident_run<double, 12, 256>(A, grid, smem, s);
+        case 13: return launch_resident_run<double, 13, 256, true>(A, grid, smem, s);
+        case 15: return launch_resident_run<double, 15, 256, true>(A, grid, smem, s);
         default: return cudaErrorInvalidValue;
     }
 }
