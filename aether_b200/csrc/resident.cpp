@@ -279,22 +279,26 @@ void aefdtd_sim::build_resident() {
                 const std::vector<int> zc = cut(wz, ns);
                 int deep = 0;
                 for (int s = 0; s < ns; s++) deep = std::max(deep, zc[s + 1] - zc[s]);
+                const double waits = nb * ns > 1 ? 2600 : 600;
+                std::vector<ResBlock> x;   // filled for the first kernel that may be better
                 for (size_t n = 0; n < nkernels; n++) {
                     const ResKernel &K = kernels[n];
                     const int runs = (deep + K.run - 1) / K.run;
                     if (Nx * tall * runs > K.threads) continue;
-                    const double waits = nb * ns > 1 ? 2600 : 600;
                     if (waits + 2 * half(tall, deep, runs, K.run, 0) >= best) continue;
                     double worst = waits;
-                    std::vector<ResBlock> x(size_t(nb) * ns);
                     bool better = true;
-                    for (int s = 0; s < ns && better; s++)
-                        for (int b = 0; b < nb && better; b++) {
-                            ResBlock &y = x[size_t(s) * nb + b];
-                            fill(y, yc[b], yc[b + 1], zc[s], zc[s + 1], K.run);
-                            worst = std::max(worst, waits + cost(y, K));
-                            better = y.disp_n < kResNoRank && worst < best && !(K.tight && ((y.feat_e | y.feat_h) & kXY));
-                        }
+                    if (x.empty()) {
+                        x.resize(size_t(nb) * ns);
+                        for (int s = 0; s < ns; s++)
+                            for (int b = 0; b < nb; b++) fill(x[size_t(s) * nb + b], yc[b], yc[b + 1], zc[s], zc[s + 1], K.run);
+                    }
+                    for (size_t m = 0; m < x.size() && better; m++) {
+                        ResBlock &y = x[m];
+                        y.nseg = (y.bz + K.run - 1) / K.run;
+                        worst = std::max(worst, waits + cost(y, K));
+                        better = y.disp_n < kResNoRank && worst < best && !(K.tight && ((y.feat_e | y.feat_h) & kXY));
+                    }
                     for (size_t m = 0; m < x.size() && better; m++) better = layout(x[m], K) <= limit;
                     if (!better) continue;
                     best = worst;
@@ -398,19 +402,23 @@ void aefdtd_sim::build_resident() {
     // planes), at least four steps, at most a segment
     const size_t room = size_t(sensors.empty() ? 8 : 64) << 20;
     res.cap = res.rec ? (int)std::clamp<size_t>(room / (res.rec * es), 4, seg_len) : seg_len;
-    auto put = [&](DBuf &b, const void *p, size_t n) {
-        b.alloc(std::max<size_t>(n, 16), dev_bytes);
-        if (n) AE_CUDA(cudaMemcpy(b.p, p, n, cudaMemcpyHostToDevice));
+    std::vector<char> host;
+    auto put = [&](const void *p, size_t n) {
+        const size_t o = host.size();
+        host.resize((o + n + 255) / 256 * 256);
+        if (n) std::memcpy(host.data() + o, p, n);
+        return o;
     };
-    put(res.blocks, B.data(), sizeof(ResBlock) * B.size());
-    put(res.disp, disp_cells.data(), sizeof(ResDisp) * disp_cells.size());
-    put(res.taps, taps.data(), sizeof(ResTaps) * taps.size());
-    put(res.sites, sites.data(), sizeof(uint2) * sites.size());
-    res.raw.alloc(std::max<size_t>(res.rec * es * res.cap, 16), dev_bytes);
-    res.inbox.alloc(std::max<size_t>(size_t(words) * 2 * es, 16), dev_bytes);
-    AE_CUDA(cudaMemsetAsync(res.inbox.p, 0, res.inbox.n, stream));
-    if (!res.abort.p) res.abort.alloc(sizeof(int), dev_bytes);
-    AE_CUDA(cudaMemsetAsync(res.abort.p, 0, sizeof(int), stream));
+    put(B.data(), sizeof(ResBlock) * B.size());
+    res.disp = put(disp_cells.data(), sizeof(ResDisp) * disp_cells.size());
+    res.taps = put(taps.data(), sizeof(ResTaps) * taps.size());
+    res.sites = put(sites.data(), sizeof(uint2) * sites.size());
+    res.inbox = host.size();
+    res.abort = res.inbox + up16(size_t(words) * 2 * es);
+    res.raw = (res.abort + 16 + 255) / 256 * 256;
+    res.mem.alloc(res.raw + res.rec * es * res.cap, dev_bytes);
+    AE_CUDA(cudaMemcpy(res.mem.p, host.data(), host.size(), cudaMemcpyHostToDevice));
+    AE_CUDA(cudaMemsetAsync(res.at<char>(res.inbox), 0, res.raw - res.inbox, stream));
     res.seq = 0;
     res.smem = (int)smem;
     res.run = run;
@@ -433,18 +441,18 @@ template <typename T> void aefdtd_sim::run_resident(int n) {
         AE_CUDA(cudaMemcpyAsync(tbl, host.data(), sizeof(StepScalars) * L, cudaMemcpyHostToDevice, stream));
         ResArgs<T> A{};
         make_step_args(A.e, A.h, tbl);
-        A.blocks = res.blocks.as<ResBlock>();
-        A.disp = res.disp.as<ResDisp>();
+        A.blocks = res.at<ResBlock>(0);
+        A.disp = res.at<ResDisp>(res.disp);
         A.npoles = (int)(crec.n / (2 * sizeof(T)));
-        A.taps = res.taps.as<ResTaps>();
-        A.sites = res.sites.as<uint2>();
-        A.inbox = res.inbox.as<unsigned long long>();
-        A.raw = res.raw.as<T>();
+        A.taps = res.at<ResTaps>(res.taps);
+        A.sites = res.at<uint2>(res.sites);
+        A.inbox = res.at<unsigned long long>(res.inbox);
+        A.raw = res.at<T>(res.raw);
         A.rec = res.rec;
         A.steps = L;
         A.seq0 = res.seq;
         res.seq += 2u * (unsigned)L + 2u;
-        A.abort = res.abort.as<int>();
+        A.abort = res.at<int>(res.abort);
         A.wait_cycles = res.wait_cycles;
         A.withhold = res.withhold;
         AE_CUDA(launch_resident(A, res.run, res.grid, res.smem, stream));
@@ -453,7 +461,7 @@ template <typename T> void aefdtd_sim::run_resident(int n) {
         if (normal) {
             SensorStepArgs<T> sa;
             make_sensor_args(sa, tbl);
-            launch_resident_planes(sa, res.raw.as<T>(), res.rec, L, stream);
+            launch_resident_planes(sa, res.at<T>(res.raw), res.rec, L, stream);
             launch_plane_reduce(psum_partial.as<double>(), sa.nbp, tbl, psums.as<double>(), L, stream);
             launches += 2;
             reg = 2;
@@ -462,7 +470,7 @@ template <typename T> void aefdtd_sim::run_resident(int n) {
             const ResRegion &r = res.region[reg++];
             if (s->nbuf == 0) s->buf_step0 = s->step;
             ResGatherArgs<T> g{};
-            g.raw = res.raw.as<T>() + r.base;
+            g.raw = res.at<T>(res.raw) + r.base;
             g.rec = res.rec;
             g.stride = r.stride;
             g.sx = r.sx; g.sy = r.sy; g.sz = r.sz;

@@ -1542,7 +1542,7 @@ void aefdtd_sim::check_err() {
         AE_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), stream));
         // a staged launch that gave up may have left its unit counters set
         if (tma_ctr.p) AE_CUDA(cudaMemsetAsync(tma_ctr.p, 0, tma_ctr.n, stream));
-        if (res.abort.p) AE_CUDA(cudaMemsetAsync(res.abort.p, 0, res.abort.n, stream));
+        if (res.mem.p) AE_CUDA(cudaMemsetAsync(res.at<int>(res.abort), 0, sizeof(int), stream));
         fail(AEFDTD_TIMEOUT, "a bounded device wait ran out");
     }
 }
@@ -1572,7 +1572,7 @@ void aefdtd_sim::zero_state() {
     for (auto &b : psiH) if (b.p) AE_CUDA(cudaMemsetAsync(b.p, 0, b.n, stream));
     if (psi.p) AE_CUDA(cudaMemsetAsync(psi.p, 0, psi.n, stream));
     if (tma_ctr.p) AE_CUDA(cudaMemsetAsync(tma_ctr.p, 0, tma_ctr.n, stream));
-    if (res.abort.p) AE_CUDA(cudaMemsetAsync(res.abort.p, 0, res.abort.n, stream));
+    if (res.mem.p) AE_CUDA(cudaMemsetAsync(res.at<int>(res.abort), 0, sizeof(int), stream));
     if (obl) {
         for (int c = 0; c < 6; c++) {
             DBuf *b[3] = {&obl->Fi[c], &obl->psiEi[c], &obl->psiHi[c]};

@@ -204,9 +204,12 @@ struct ResidentPlan {
     unsigned seq = 0;              // half-steps numbered so far on the inboxes
     long long wait_cycles = 1LL << 31;   // bound of each wait, and the test hook (aefdtd_test_hook)
     int withhold = 0;
-    DBuf blocks, disp, taps, sites, raw, inbox, abort;
+    // one allocation: blocks, dispersive cells, taps, sites, inboxes, the abort word, records
+    DBuf mem;
+    size_t disp = 0, taps = 0, sites = 0, inbox = 0, abort = 0, raw = 0;   // their byte offsets
+    template <typename U> U *at(size_t offset) const { return reinterpret_cast<U *>(static_cast<char *>(mem.p) + offset); }
     void release(size_t &t) {
-        for (DBuf *b : {&blocks, &disp, &taps, &sites, &raw, &inbox, &abort}) b->release(t);
+        mem.release(t);
         grid = 0;
     }
 };
