@@ -1242,6 +1242,13 @@ void aefdtd_sim::build_work() {
         long long want = 148LL * 12 * 3;
         kchunk = 8;
         while (kchunk > 4 && tiles * ((Nz + kchunk - 1) / kchunk) < want) kchunk /= 2;
+        // The FP32 pair kernels of a grid that stays in L2 (up to 110 MB of
+        // fields) take 3: a shorter chain of planes, and reading the plane
+        // below again costs L2 only. us per step with 4 and 3 planes:
+        // 80x80x200 27.0 / 26.1, 120x120x200 44.8 / 43.1, 128x128x128
+        // 30.5 / 29.3, 128x128x256 66.5 / 65.8; past L2 150x140x250
+        // 84.4 / 85.1. FP64 pairs and single cells are slower with 3.
+        if (kchunk == 4 && !fp64 && pmask && 24.0 * Nx * Ny * Nz <= 110e6) kchunk = 3;
     }
     const int nch = (Nz + kchunk - 1) / kchunk;
     // feature mask per (tile, plane) (kF* of yee.cuh); oscillator boxes matter to E only
