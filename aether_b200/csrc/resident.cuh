@@ -17,9 +17,9 @@
 // measured 9.0 us against 5.6 us per step on a 40 x 40 x 200 FP32 cell; the
 // split half-steps take 13.8 us.) CPML psi of z is in shared memory, psi of x
 // and y and the recursive-convolution psi (18 values per cell for three poles)
-// in global
-// memory; the latter's update reads only the block's own E and runs before
-// the block waits for its neighbours.
+// in global memory; the latter's update reads only the block's own E and runs
+// before the block waits for its neighbours. The longest runs share one array
+// between E and H (Tight).
 //
 // Exchange. An E update needs H of the y-1 and z-1 blocks, an H update E of
 // the y+1 and z+1 blocks (fdtd_core.cpp:363-969; both wrap). The thread that
@@ -42,9 +42,10 @@
 // Bound: per half-step the slowest block's issue slots (about 12 cycles per
 // warp and plane in FP32, 20 in FP64, twice that in a z-CPML slab) and one
 // inbox round trip of 1000 to 1300 cycles. Measured per step, resident against
-// split: 12 x 10 x 90 FP64 4.3 / 13.4 us, 48 x 48 x 128 FP64 7.5 / 16.2,
-// 40 x 40 x 200 FP32 5.6 / 13.8, 64 x 64 x 128 FP32 with two 61-wavelength flux
-// planes 8.3 / 15.1.
+// split: 12 x 10 x 90 FP64 4.5 / 13.5 us, 48 x 48 x 128 FP64 7.6 / 16.2,
+// 64 x 64 x 128 FP64 12.6 / 20.0, 40 x 40 x 200 FP32 with a disk of poles
+// 5.9 / 13.9, 64 x 64 x 128 FP32 with two 61-wavelength flux planes 8.4 / 15.1,
+// 64 x 64 x 250 FP32 11.6 / 17.8.
 #pragma once
 
 #include <cuda_runtime.h>
