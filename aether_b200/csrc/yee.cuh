@@ -307,7 +307,7 @@ __device__ __forceinline__ T bloch_ghost(int bloch, T own, T other, double c, do
 }
 
 // ---- boundary items: the phases of feature set F ---------------------------
-template <typename T, typename Tid, unsigned F, bool Coh = false>
+template <typename T, typename Tid, unsigned F, bool Coh = false, int U = 1>
 __device__ __forceinline__ void e_boundary_body(const StepArgs<T, Tid> &a, int q, int4 it) {
     const int i = it.x + threadIdx.x, j = it.y + threadIdx.y;
     if (i >= a.Nx || j >= a.Ny) return;
@@ -372,11 +372,43 @@ __device__ __forceinline__ void e_boundary_body(const StepArgs<T, Tid> &a, int q
     T hx_km = ldf<Coh>(Hx + col + kmi * NxNy);
     T hy_km = ldf<Coh>(Hy + col + kmi * NxNy);
 
-    for (int k = k0; k < k1; ++k) {
+    for (int kb = k0; kb < k1; kb += U) {
+      struct { T hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, ex, ey, ez, qy0, qy1, qx0, qx1, qz0, qz1; int m; } in[U];
+      // the plane's psi, every value loaded before any is stored (the six arrays are distinct)
+      const auto load_psi = [&](int u, int k) {
+          in[u].qy0 = in[u].qy1 = in[u].qx0 = in[u].qx1 = in[u].qz0 = in[u].qz1 = 0;
+          if constexpr ((F & kFPmlXY) != 0) {
+              const long long oy = i + (long long)yn * a.Nx + (long long)k * a.Nx * nys;
+              const long long ox = xn + (long long)j * nxs + (long long)k * nxs * a.Ny;
+              if (ye) { in[u].qy0 = a.psi_y0[oy]; in[u].qy1 = a.psi_y1[oy]; }
+              if (xe) { in[u].qx0 = a.psi_x0[ox]; in[u].qx1 = a.psi_x1[ox]; }
+          }
+          if constexpr ((F & kFPmlZ) != 0) {
+              if (a.pz && ((k >= 1 && k < a.pml_zm) || (k >= a.Nz - a.pml_zp + 1))) {
+                  const long long oz = col + (long long)((k < a.pml_zm) ? k : k - (a.Nz - a.pml_zp) + a.pml_zm) * NxNy;
+                  in[u].qz0 = a.psi_z0[oz]; in[u].qz1 = a.psi_z1[oz];
+              }
+          }
+      };
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = kb + u;
+        if (U > 1 && k >= k1) continue;
         const long long id = col + k * NxNy;
-        const T hx = ldf<Coh>(Hx + id), hy = ldf<Coh>(Hy + id), hz = ldf<Coh>(Hz + id);
-        T hz_jm = ldf<Coh>(Hz + coly + k * NxNy), hx_jm = ldf<Coh>(Hx + coly + k * NxNy);
-        T hz_im = ldf<Coh>(Hz + colx + k * NxNy), hy_im = ldf<Coh>(Hy + colx + k * NxNy);
+        in[u].hx = ldf<Coh>(Hx + id); in[u].hy = ldf<Coh>(Hy + id); in[u].hz = ldf<Coh>(Hz + id);
+        in[u].hz_jm = ldf<Coh>(Hz + coly + k * NxNy); in[u].hx_jm = ldf<Coh>(Hx + coly + k * NxNy);
+        in[u].hz_im = ldf<Coh>(Hz + colx + k * NxNy); in[u].hy_im = ldf<Coh>(Hy + colx + k * NxNy);
+        in[u].ex = Ex[id]; in[u].ey = Ey[id]; in[u].ez = Ez[id];
+        in[u].m = __ldg(a.mat + colm + k * mNxNy);
+        if constexpr (U > 1) load_psi(u, k);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = kb + u;
+        if (U > 1 && k >= k1) continue;
+        const long long id = col + k * NxNy;
+        const T hx = in[u].hx, hy = in[u].hy, hz = in[u].hz;
+        T hz_jm = in[u].hz_jm, hx_jm = in[u].hx_jm, hz_im = in[u].hz_im, hy_im = in[u].hy_im;
         if constexpr ((F & kFMisc) != 0) {
             // oblique driver: H ghosts past the y = 0 and x = 0 edges (set before update_E)
             if (a.bloch) {
@@ -390,8 +422,8 @@ __device__ __forceinline__ void e_boundary_body(const StepArgs<T, Tid> &a, int q
                 }
             }
         }
-        const T ex = Ex[id], ey = Ey[id], ez = Ez[id];
-        const int m = __ldg(a.mat + colm + k * mNxNy);
+        const T ex = in[u].ex, ey = in[u].ey, ez = in[u].ez;
+        const int m = in[u].m;
         const MatCoef<T> c = a.coef[m];
         const T ikz = __ldg(a.ikz + k);
 
@@ -458,9 +490,7 @@ __device__ __forceinline__ void e_boundary_body(const StepArgs<T, Tid> &a, int q
             }
         }
 
-        // CPML and PEC planes in app_pml_Ex / Ey / Ez order. Every psi value the
-        // cell needs is loaded before any is stored (the six arrays are distinct),
-        // so the loads are in flight together.
+        // CPML and PEC planes in app_pml_Ex / Ey / Ez order
         bool ze = false;
         int zn = 0;
         T bzk = 0, czk = 0;
@@ -472,14 +502,8 @@ __device__ __forceinline__ void e_boundary_body(const StepArgs<T, Tid> &a, int q
         const long long oy = i + (long long)yn * a.Nx + (long long)k * a.Nx * nys;
         const long long ox = xn + (long long)j * nxs + (long long)k * nxs * a.Ny;
         const long long oz = col + (long long)zn * NxNy;
-        T qy0 = 0, qy1 = 0, qx0 = 0, qx1 = 0, qz0 = 0, qz1 = 0;
-        if constexpr ((F & kFPmlXY) != 0) {
-            if (ye) { qy0 = a.psi_y0[oy]; qy1 = a.psi_y1[oy]; }
-            if (xe) { qx0 = a.psi_x0[ox]; qx1 = a.psi_x1[ox]; }
-        }
-        if constexpr ((F & kFPmlZ) != 0) {
-            if (ze) { qz0 = a.psi_z0[oz]; qz1 = a.psi_z1[oz]; }
-        }
+        if constexpr (U == 1) load_psi(u, k);
+        const T qy0 = in[u].qy0, qy1 = in[u].qy1, qx0 = in[u].qx0, qx1 = in[u].qx1, qz0 = in[u].qz0, qz1 = in[u].qz1;
         // Ex: y block, then z block
         if constexpr ((F & kFPmlXY) != 0) {
             if (ye) {
@@ -563,10 +587,11 @@ __device__ __forceinline__ void e_boundary_body(const StepArgs<T, Tid> &a, int q
         Ez[id] = nez;
         hx_km = hx;
         hy_km = hy;
+      }
     }
 }
 
-template <typename T, typename Tid, unsigned F, bool Coh = false>
+template <typename T, typename Tid, unsigned F, bool Coh = false, int U = 1>
 __device__ __forceinline__ void h_boundary_body(const StepArgs<T, Tid> &a, int q, int4 it) {
     const int i = it.x + threadIdx.x, j = it.y + threadIdx.y;
     if (i >= a.Nx || j >= a.Ny) return;
@@ -627,13 +652,44 @@ __device__ __forceinline__ void h_boundary_body(const StepArgs<T, Tid> &a, int q
     T ex = ldf<Coh>(Ex + col + k0 * NxNy);
     T ey = ldf<Coh>(Ey + col + k0 * NxNy);
 
-    for (int k = k0; k < k1; ++k) {
+    for (int kb = k0; kb < k1; kb += U) {
+      struct { T ex_kp, ey_kp, ez, ez_jp, ex_jp, ez_ip, ey_ip, hx, hy, hz, qy0, qy1, qx0, qx1, qz0, qz1; } in[U];
+      // the plane's psi, every load before any store (distinct arrays)
+      const auto load_psi = [&](int u, int k) {
+          in[u].qy0 = in[u].qy1 = in[u].qx0 = in[u].qx1 = in[u].qz0 = in[u].qz1 = 0;
+          if constexpr ((F & kFPmlXY) != 0) {
+              const long long oy = i + (long long)yn * a.Nx + (long long)k * a.Nx * nys;
+              const long long ox = xn + (long long)j * nxs + (long long)k * nxs * a.Ny;
+              if (yh) { in[u].qy0 = a.psi_y0[oy]; in[u].qy1 = a.psi_y1[oy]; }
+              if (xh) { in[u].qx0 = a.psi_x0[ox]; in[u].qx1 = a.psi_x1[ox]; }
+          }
+          if constexpr ((F & kFPmlZ) != 0) {
+              if (a.pz && ((k < a.pml_zm) || (k >= a.Nz - a.pml_zp && k < a.Nz - 1))) {
+                  const long long oz = col + (long long)((k < a.pml_zm) ? k : k - (a.Nz - a.pml_zp) + a.pml_zm) * NxNy;
+                  in[u].qz0 = a.psi_z0[oz]; in[u].qz1 = a.psi_z1[oz];
+              }
+          }
+      };
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = kb + u;
+        if (U > 1 && k >= k1) continue;
         const long long id = col + k * NxNy;
         const int kp = (k == a.Nz - 1) ? 0 : k + 1;
-        const T ex_kp = ldf<Coh>(Ex + col + kp * NxNy), ey_kp = ldf<Coh>(Ey + col + kp * NxNy);
-        const T ez = ldf<Coh>(Ez + id);
-        T ez_jp = ldf<Coh>(Ez + coly + k * NxNy), ex_jp = ldf<Coh>(Ex + coly + k * NxNy);
-        T ez_ip = ldf<Coh>(Ez + colx + k * NxNy), ey_ip = ldf<Coh>(Ey + colx + k * NxNy);
+        in[u].ex_kp = ldf<Coh>(Ex + col + kp * NxNy); in[u].ey_kp = ldf<Coh>(Ey + col + kp * NxNy);
+        in[u].ez = ldf<Coh>(Ez + id);
+        in[u].ez_jp = ldf<Coh>(Ez + coly + k * NxNy); in[u].ex_jp = ldf<Coh>(Ex + coly + k * NxNy);
+        in[u].ez_ip = ldf<Coh>(Ez + colx + k * NxNy); in[u].ey_ip = ldf<Coh>(Ey + colx + k * NxNy);
+        in[u].hx = Hx[id]; in[u].hy = Hy[id]; in[u].hz = Hz[id];
+        if constexpr (U > 1) load_psi(u, k);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = kb + u;
+        if (U > 1 && k >= k1) continue;
+        const long long id = col + k * NxNy;
+        const T ex_kp = in[u].ex_kp, ey_kp = in[u].ey_kp, ez = in[u].ez;
+        T ez_jp = in[u].ez_jp, ex_jp = in[u].ex_jp, ez_ip = in[u].ez_ip, ey_ip = in[u].ey_ip;
         if constexpr ((F & kFMisc) != 0) {
             // oblique driver: E ghosts past the y = Ny-1 and x = Nx-1 edges (set after inject_E)
             if (a.bloch) {
@@ -647,7 +703,7 @@ __device__ __forceinline__ void h_boundary_body(const StepArgs<T, Tid> &a, int q
                 }
             }
         }
-        const T hx = Hx[id], hy = Hy[id], hz = Hz[id];
+        const T hx = in[u].hx, hy = in[u].hy, hz = in[u].hz;
         const T az = a.dtdmz * __ldg(a.ikz + k);
 
         const T dEy_z = ey_kp - ey, dEz_y = ez_jp - ez;
@@ -665,18 +721,11 @@ __device__ __forceinline__ void h_boundary_body(const StepArgs<T, Tid> &a, int q
             zn = (k < a.pml_zm) ? k : k - (a.Nz - a.pml_zp) + a.pml_zm;
             if (zh) { bzk = __ldg(a.bz + k); czk = __ldg(a.cz + k); }
         }
-        // every psi load of the cell before any store (distinct arrays)
         const long long oy = i + (long long)yn * a.Nx + (long long)k * a.Nx * nys;
         const long long ox = xn + (long long)j * nxs + (long long)k * nxs * a.Ny;
         const long long oz = col + (long long)zn * NxNy;
-        T qy0 = 0, qy1 = 0, qx0 = 0, qx1 = 0, qz0 = 0, qz1 = 0;
-        if constexpr ((F & kFPmlXY) != 0) {
-            if (yh) { qy0 = a.psi_y0[oy]; qy1 = a.psi_y1[oy]; }
-            if (xh) { qx0 = a.psi_x0[ox]; qx1 = a.psi_x1[ox]; }
-        }
-        if constexpr ((F & kFPmlZ) != 0) {
-            if (zh) { qz0 = a.psi_z0[oz]; qz1 = a.psi_z1[oz]; }
-        }
+        if constexpr (U == 1) load_psi(u, k);
+        const T qy0 = in[u].qy0, qy1 = in[u].qy1, qx0 = in[u].qx0, qx1 = in[u].qx1, qz0 = in[u].qz0, qz1 = in[u].qz1;
         // Hx: y block, then z block
         if constexpr ((F & kFPmlXY) != 0) {
             if (yh) {
@@ -749,6 +798,7 @@ __device__ __forceinline__ void h_boundary_body(const StepArgs<T, Tid> &a, int q
         Hz[id] = nhz;
         ex = ex_kp;
         ey = ey_kp;
+      }
     }
 }
 
@@ -1132,6 +1182,23 @@ __global__ void __launch_bounds__(kMaxTileThreads) h_boundary(const __grid_const
     h_boundary_body<T, Tid, F>(a, a.q, items[blockIdx.x]);
 }
 
+// CPML items with x-CPML cells: bound by the round trip per plane (ncu: long
+// scoreboard 9.6 of the stalls at 0.43 of the DRAM rate, one plane at a time).
+// A column's planes need no result of each other, so the loads of two planes are
+// issued together. us per half-step of all x/y-CPML items, one / two / three
+// planes: 384x384x192 FP64 E 235 / 220 / 261, H 232 / 211 / 237; 768x768x384
+// FP32 E 537 / 517 / 549, H 473 / 481 / 525, so the FP32 H keeps one.
+template <typename T, typename Tid>
+__global__ void __launch_bounds__(kMaxTileThreads, sizeof(T) == 8 ? 2 : 3) e_pmlx(const __grid_constant__ StepArgs<T, Tid> a,
+                                                                                  const int4 *__restrict__ items) {
+    e_boundary_body<T, Tid, kFPmlXY | kFPmlZ, false, 2>(a, a.q, items[blockIdx.x]);
+}
+template <typename T, typename Tid>
+__global__ void __launch_bounds__(kMaxTileThreads, sizeof(T) == 8 ? 2 : 4) h_pmlx(const __grid_constant__ StepArgs<T, Tid> a,
+                                                                                  const int4 *__restrict__ items) {
+    h_boundary_body<T, Tid, kFPmlXY | kFPmlZ, false, (sizeof(T) == 8 ? 2 : 1)>(a, a.q, items[blockIdx.x]);
+}
+
 template <typename T, typename Tid, bool PZ>
 __global__ void __launch_bounds__(kMaxTileThreads, InteriorBounds<T, 2, PZ>::kMinBlocksVec2)
 e_interior_v2(const __grid_constant__ StepArgs<T, Tid> a, const int4 *__restrict__ items) {
@@ -1212,7 +1279,7 @@ void launch_e_group_impl(const StepArgs<T, Tid> &a, const int4 *items, const Wor
         case kGroupDisp: e_boundary<T, Tid, kFDisp><<<n, blk, 0, s>>>(a, p); break;
         case kGroupPmlXY:
             // items with x-CPML cells first (one cell per thread), then the y-only pairs
-            if (n > w.n_py) e_boundary<T, Tid, kFPmlXY | kFPmlZ><<<n - w.n_py, blk, 0, s>>>(a, p);
+            if (n > w.n_py) e_pmlx<T, Tid><<<n - w.n_py, blk, 0, s>>>(a, p);
             if (w.n_py > 0) e_pmly_v2<T, Tid><<<w.n_py, blk, 0, s>>>(a, p + (n - w.n_py));
             break;
         default: e_boundary<T, Tid, kFAll><<<n, blk, 0, s>>>(a, p); break;
@@ -1238,7 +1305,7 @@ void launch_h_group_impl(const StepArgs<T, Tid> &a, const int4 *items, const Wor
             else h_interior<T, Tid, 1, true><<<n, blk, 0, s>>>(a, p);
             break;
         case kGroupPmlXY:
-            if (n > w.n_py) h_boundary<T, Tid, kFPmlXY | kFPmlZ><<<n - w.n_py, blk, 0, s>>>(a, p);
+            if (n > w.n_py) h_pmlx<T, Tid><<<n - w.n_py, blk, 0, s>>>(a, p);
             if (w.n_py > 0) h_pmly_v2<T, Tid><<<w.n_py, blk, 0, s>>>(a, p + (n - w.n_py));
             break;
         default: h_boundary<T, Tid, kFAll><<<n, blk, 0, s>>>(a, p); break;
