@@ -26,8 +26,9 @@
 //     each thread keeps U planes of reads in flight;
 //   * z-CPML items: the same loop with the psi_z recursions and z PEC planes
 //     (PZ instantiation of the interior kernels);
-//   * x/y-CPML items (with or without z-CPML): the boundary kernel for
-//     kFPmlXY | kFPmlZ (about 50 registers instead of 120);
+//   * x/y-CPML items (with or without z-CPML): with x-CPML cells the boundary
+//     body for kFPmlXY | kFPmlZ, two planes at a time (e_pmlx, h_pmlx), else
+//     two cells per thread (e_pmly_v2, h_pmly_v2);
 //   * dispersive items and the rest (every phase): the boundary kernel
 //     instantiated for feature sets kFDisp and kFAll.
 // All groups of a half-step together cover each cell exactly once.
