@@ -394,7 +394,8 @@ struct FluxArgs {
     int P, nl, type;
     double area_factor;      // Dy*Dz, Dx*Dz or Dx*Dy
     const double2 *acc;      // [6][nl][P]
-    double *out;             // nl
+    double *out;             // nl, and behind them the error flag
+    const int *err;
 };
 
 // Tensor-core DFT (dft_tc.cu). B image: per tile [E hi, E lo, H hi, H lo] of

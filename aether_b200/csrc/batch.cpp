@@ -1064,6 +1064,7 @@ aefdtd_status aefdtd_batch_add(aefdtd_batch *b, aefdtd_sim *s, int32_t steps) {
         if (!s->sensors.empty()) fail(AEFDTD_BAD_ARG, "batch members carry no planar DFT sensors (normal-mode plane sums only)");
         if (!s->fmaps.empty()) fail(AEFDTD_BAD_ARG, "batch members carry no field sensors");
         if (s->Nz >= 32768) fail(AEFDTD_BAD_ARG, "batch members need Nz < 32768 (k1 << 16 in an int32 item)");
+        s->check_state();
         s->set_device();
         s->finalize_tables();
         s->tma_allowed = false;      // merged lists take every interior item
@@ -1078,7 +1079,7 @@ aefdtd_status aefdtd_batch_add(aefdtd_batch *b, aefdtd_sim *s, int32_t steps) {
         } else if (s->fp64 != b->fp64 || s->id_bytes != b->id_bytes || s->seg_len != b->seg_len) {
             fail(AEFDTD_BAD_ARG, "batch members share precision, material-id width and DFT block");
         }
-        AE_CUDA(cudaStreamSynchronize(s->stream));
+        s->check_err();
         BatchMember m;
         m.sim = s;
         m.remaining = (s->cc_coeff > 0 && s->cc_done) ? 0 : steps;

@@ -414,8 +414,7 @@ void aefdtd_sim::build_resident() {
     res.taps = put(taps.data(), sizeof(ResTaps) * taps.size());
     res.sites = put(sites.data(), sizeof(uint2) * sites.size());
     res.inbox = host.size();
-    res.abort = res.inbox + up16(size_t(words) * 2 * es);
-    res.raw = (res.abort + 16 + 255) / 256 * 256;
+    res.raw = (res.inbox + up16(size_t(words) * 2 * es) + 255) / 256 * 256;
     res.mem.alloc(res.raw + res.rec * es * res.cap, dev_bytes);
     AE_CUDA(cudaMemcpy(res.mem.p, host.data(), host.size(), cudaMemcpyHostToDevice));
     AE_CUDA(cudaMemsetAsync(res.at<char>(res.inbox), 0, res.raw - res.inbox, stream));
@@ -452,7 +451,7 @@ template <typename T> void aefdtd_sim::run_resident(int n) {
         A.steps = L;
         A.seq0 = res.seq;
         res.seq += 2u * (unsigned)L + 2u;
-        A.abort = res.at<int>(res.abort);
+        A.abort = err.as<int>() + 1;
         A.wait_cycles = res.wait_cycles;
         A.withhold = res.withhold;
         AE_CUDA(launch_resident(A, res.run, res.grid, res.smem, stream));

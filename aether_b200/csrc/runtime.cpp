@@ -112,8 +112,8 @@ void aefdtd_sim::construct(const aefdtd_grid_desc *d) {
     seg_len = dft_k;
     tables.alloc(sizeof(StepScalars) * 2 * seg_len, dev_bytes);
     if (std::getenv("AEFDTD_NO_GRAPHS")) use_graphs = false;
-    err.alloc(sizeof(int), dev_bytes);
-    AE_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), stream));
+    err.alloc(2 * sizeof(int), dev_bytes);
+    AE_CUDA(cudaMemsetAsync(err.p, 0, err.n, stream));
     map.assign(N, 0);
     Nmat = 1;
     mats.assign(1, HostMat());
@@ -1540,18 +1540,24 @@ void aefdtd_sim::build_work() {
     work_dirty = false;
 }
 
-// Reads the device error flag set by a bounded wait that ran out.
+// Reads the device error flag set by a bounded wait that ran out. Every call
+// that hands out results ends with it: what such a launch left is no result.
 void aefdtd_sim::check_err() {
-    int h = 0;
-    AE_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    int h[2] = {0, 0};
+    AE_CUDA(cudaMemcpyAsync(h, err.p, sizeof(h), cudaMemcpyDeviceToHost, stream));
     AE_CUDA(cudaStreamSynchronize(stream));
-    if (h) {
-        AE_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), stream));
+    if (h[0]) {
+        AE_CUDA(cudaMemsetAsync(err.p, 0, err.n, stream));
         // a staged launch that gave up may have left its unit counters set
         if (tma_ctr.p) AE_CUDA(cudaMemsetAsync(tma_ctr.p, 0, tma_ctr.n, stream));
-        if (res.mem.p) AE_CUDA(cudaMemsetAsync(res.at<int>(res.abort), 0, sizeof(int), stream));
+        // a resident launch that gave up kept its fields and not its psi: only a reset mends that
+        lost |= h[1] != 0;
         fail(AEFDTD_TIMEOUT, "a bounded device wait ran out");
     }
+}
+
+void aefdtd_sim::check_state() const {
+    if (lost) fail(AEFDTD_TIMEOUT, "a resident launch ran out of a bounded wait: reset the simulation first");
 }
 
 void aefdtd_sim::step(int n) {
@@ -1559,6 +1565,7 @@ void aefdtd_sim::step(int n) {
     if (!map_set) fail(AEFDTD_NOT_READY, "no material map");
     if (g.mode == AEFDTD_MODE_NORMAL && !normal) fail(AEFDTD_NOT_READY, "normal mode needs aefdtd_setup_normal");
     if (g.mode == AEFDTD_MODE_OBLIQUE && !obl) fail(AEFDTD_NOT_READY, "oblique mode needs aefdtd_setup_oblique");
+    check_state();
     set_device();
     finalize_tables();
     if (fp64) {
@@ -1579,7 +1586,9 @@ void aefdtd_sim::zero_state() {
     for (auto &b : psiH) if (b.p) AE_CUDA(cudaMemsetAsync(b.p, 0, b.n, stream));
     if (psi.p) AE_CUDA(cudaMemsetAsync(psi.p, 0, psi.n, stream));
     if (tma_ctr.p) AE_CUDA(cudaMemsetAsync(tma_ctr.p, 0, tma_ctr.n, stream));
-    if (res.mem.p) AE_CUDA(cudaMemsetAsync(res.at<int>(res.abort), 0, sizeof(int), stream));
+    // a wait that ran out before is no fault of the steps to come
+    AE_CUDA(cudaMemsetAsync(err.p, 0, err.n, stream));
+    lost = false;
     if (obl) {
         for (int c = 0; c < 6; c++) {
             DBuf *b[3] = {&obl->Fi[c], &obl->psiEi[c], &obl->psiHi[c]};
@@ -1762,7 +1771,7 @@ aefdtd_status aefdtd_add_planar_sensor(aefdtd_sim *s, const aefdtd_sensor_desc *
             p->wdev.alloc(size_t(p->nl) * 8, s->dev_bytes);
             p->WE.alloc(size_t(s->dft_k) * p->nl * 16, s->dev_bytes);
             p->WH.alloc(size_t(s->dft_k) * p->nl * 16, s->dev_bytes);
-            p->flux.alloc(size_t(p->nl) * 8, s->dev_bytes);
+            p->flux.alloc(size_t(p->nl + 1) * 8, s->dev_bytes);
             AE_CUDA(cudaMemsetAsync(p->acc.p, 0, p->acc.n, s->stream));
             AE_CUDA(cudaMemsetAsync(p->S.p, 0, p->S.n, s->stream));
             // FP32 path: DFT blocks on the tensor cores when K is a multiple of 8
@@ -1827,6 +1836,7 @@ aefdtd_status aefdtd_get_field(aefdtd_sim *s, int32_t c, double *out, size_t cou
         if (c < 0 || c > (s->obl ? 11 : 5)) fail(AEFDTD_BAD_ARG, "component out of range");
         size_t N = size_t(s->Nx) * s->Ny * s->Nz;
         if (count != N) fail(AEFDTD_BAD_ARG, "count must be Nx*Ny*Nz of the total grid");
+        s->check_state();
         s->set_device();
         const void *src = s->grid_fields(c / 6)[c % 6].p;
         if (s->fp64) {
@@ -1838,6 +1848,7 @@ aefdtd_status aefdtd_get_field(aefdtd_sim *s, int32_t c, double *out, size_t cou
             AE_CUDA(cudaStreamSynchronize(s->stream));
             for (size_t q = 0; q < N; q++) out[q] = tmp[q];
         }
+        s->check_err();
     });
 }
 
@@ -1870,11 +1881,12 @@ aefdtd_status aefdtd_get_plane_sums(aefdtd_sim *s, double *out, int32_t steps) {
     return guarded(s, [&] {
         if (!s->normal) fail(AEFDTD_NOT_READY, "plane sums exist in normal mode only");
         if (steps != s->tstep) fail(AEFDTD_BAD_ARG, "steps must equal the number of completed steps");
+        s->check_state();
         s->set_device();
         std::vector<double> tmp(size_t(steps) * 12);
         if (steps > 0) {
             AE_CUDA(cudaMemcpyAsync(tmp.data(), s->psums.p, tmp.size() * 8, cudaMemcpyDeviceToHost, s->stream));
-            AE_CUDA(cudaStreamSynchronize(s->stream));
+            s->check_err();
         }
         for (int c = 0; c < 12; c++)
             for (int t = 0; t < steps; t++) out[size_t(c) * steps + t] = tmp[size_t(t) * 12 + c];
@@ -2110,7 +2122,8 @@ aefdtd_status aefdtd_get_fieldmap(aefdtd_sim *s, int32_t id, double *out, size_t
         else want = size_t(m.ncomp) * m.dev.P * 2;
         if (count != want) fail(AEFDTD_BAD_ARG, "count must be " + std::to_string(want));
         s->set_device();
-        AE_CUDA(cudaStreamSynchronize(s->stream));
+        s->check_state();
+        s->check_err();
         if (want) AE_CUDA(cudaMemcpy(out, m.acc.p, want * sizeof(double), cudaMemcpyDeviceToHost));
     });
 }
@@ -2129,15 +2142,20 @@ aefdtd_status aefdtd_get_sensor_flux(aefdtd_sim *s, int32_t id, double *out, int
         if (id < 0 || id >= (int)s->sensors.size()) fail(AEFDTD_BAD_ARG, "unknown sensor");
         PlaneSensor &p = *s->sensors[id];
         if (nl != p.nl) fail(AEFDTD_BAD_ARG, "nl must equal the sensor's spectrum size");
+        s->check_state();
         s->set_device();
         s->drain_sensors();
         double af = p.type <= 1 ? s->Dy * s->Dz : (p.type <= 3 ? s->Dx * s->Dz : s->Dx * s->Dy);
-        FluxArgs fa{p.P, p.nl, p.type, af, p.acc.as<double2>(), p.flux.as<double>()};
+        FluxArgs fa{p.P, p.nl, p.type, af, p.acc.as<double2>(), p.flux.as<double>(), s->err.as<int>()};
         launch_flux(fa, s->stream);
         s->launches++;
-        AE_CUDA(cudaMemcpyAsync(out, p.flux.p, size_t(nl) * 8, cudaMemcpyDeviceToHost, s->stream));
+        // the error flag travels behind the spectrum: a copy of its own costs a round trip
+        std::vector<double> tmp(size_t(nl) + 1);
+        AE_CUDA(cudaMemcpyAsync(tmp.data(), p.flux.p, tmp.size() * 8, cudaMemcpyDeviceToHost, s->stream));
         AE_CUDA(cudaStreamSynchronize(s->stream));
         AE_CUDA(cudaGetLastError());
+        if (tmp[nl] != 0) s->check_err();
+        std::memcpy(out, tmp.data(), size_t(nl) * 8);
     });
 }
 
@@ -2147,10 +2165,11 @@ aefdtd_status aefdtd_get_sensor_dft(aefdtd_sim *s, int32_t id, double *out, size
         if (id < 0 || id >= (int)s->sensors.size()) fail(AEFDTD_BAD_ARG, "unknown sensor");
         PlaneSensor &p = *s->sensors[id];
         if (count != size_t(6) * p.P * p.nl * 2) fail(AEFDTD_BAD_ARG, "count must be 6*span1*span2*nl*2");
+        s->check_state();
         s->set_device();
         s->drain_sensors();
         AE_CUDA(cudaMemcpyAsync(out, p.acc.p, count * 8, cudaMemcpyDeviceToHost, s->stream));
-        AE_CUDA(cudaStreamSynchronize(s->stream));
+        s->check_err();
     });
 }
 

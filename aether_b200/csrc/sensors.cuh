@@ -657,6 +657,7 @@ __global__ void __launch_bounds__(256) flux_reduce(FluxArgs a) {
             case 5: r = -Sz; break;
         }
         a.out[l] = r;
+        if (l == 0) a.out[a.nl] = *a.err;
     }
 }
 

@@ -204,9 +204,9 @@ struct ResidentPlan {
     unsigned seq = 0;              // half-steps numbered so far on the inboxes
     long long wait_cycles = 1LL << 31;   // bound of each wait, and the test hook (aefdtd_test_hook)
     int withhold = 0;
-    // one allocation: blocks, dispersive cells, taps, sites, inboxes, the abort word, records
+    // one allocation: blocks, dispersive cells, taps, sites, inboxes, records
     DBuf mem;
-    size_t disp = 0, taps = 0, sites = 0, inbox = 0, abort = 0, raw = 0;   // their byte offsets
+    size_t disp = 0, taps = 0, sites = 0, inbox = 0, raw = 0;   // their byte offsets
     template <typename U> U *at(size_t offset) const { return reinterpret_cast<U *>(static_cast<char *>(mem.p) + offset); }
     void release(size_t &t) {
         mem.release(t);
@@ -319,8 +319,10 @@ struct aefdtd_sim {
     DBuf items;
     std::vector<int> items_host;    // host copy of `items` (merged into batch work lists)
     void build_work();
-    DBuf err;
+    DBuf err;                // [0] a bounded wait ran out; [1] one of a resident launch did (resident.cuh)
     void check_err();
+    bool lost = false;       // a resident launch ran out of a wait: the state is undefined until a reset
+    void check_state() const;
     // timing: one event quadruple per step of the last aefdtd_step call
     // (before E, after E, after H, after sensors), summed on query
     bool timing = false;

@@ -459,8 +459,10 @@ aefdtd_status aefdtd_probe_copy_bandwidth(int32_t device, size_t bytes, int32_t 
  * and shared memory, taken when it fits): the bound of each wait for a
  * neighbour block's values (default 2^31 cycles), and (value 1) a launch whose
  * first block never updates H, so that its neighbours' waits run out; every
- * CTA then leaves at its next barrier and the next synchronising call returns
- * AEFDTD_TIMEOUT (reset the simulation before reuse). */
+ * CTA then leaves at its next barrier. The next call that synchronises or reads
+ * results returns AEFDTD_TIMEOUT, and from then on aefdtd_step and the reading
+ * calls do so until aefdtd_reset: fields and CPML state no longer belong to one
+ * step. */
 #define AEFDTD_TEST_RESIDENT_WAIT_CYCLES 7
 #define AEFDTD_TEST_RESIDENT_WITHHOLD 8
 aefdtd_status aefdtd_test_hook(aefdtd_sim *sim, int32_t what, int64_t value);

@@ -1,0 +1,56 @@
+"""Resident time steps (resident.cuh) beside the normal run: a wait that runs
+out and how it is reported."""
+import numpy as np
+import pytest
+
+from aether_b200 import _abi as A
+from aether_b200 import fdtd
+from test_resident import SCENES, WAIT_CYCLES, WITHHOLD, run
+
+pytestmark = pytest.mark.gpu
+TIMEOUT = 3   # AEFDTD_TIMEOUT
+
+
+def withhold(s, on):
+    """Launches whose first block never sends H; waits end after 2^20 cycles."""
+    assert s._lib.aefdtd_test_hook(s._h, WAIT_CYCLES, 1 << 20 if on else 1 << 31) == 0
+    assert s._lib.aefdtd_test_hook(s._h, WITHHOLD, int(on)) == 0
+
+
+READS = {"fields": lambda s: s.fields(), "sums": lambda s: s.plane_sums(), "spectra": lambda s: s.normal_spectra(),
+         "flux": lambda s: s.sensor_flux(1), "dft": lambda s: s.sensor_dft(0), "synchronize": lambda s: s.synchronize()}
+
+
+@pytest.mark.parametrize("read", sorted(READS))
+def test_a_wait_that_runs_out_is_reported_by_the_call_that_reads(read):
+    """No call hands out what an aborted launch left, whichever comes first;
+    steps and reads are refused until the reset, which mends the handle."""
+    scene = SCENES["cell"](precision=A.FP64)
+    want = run(scene, True, (40,))["fields"]
+    with fdtd.build_simulation(scene) as s:
+        withhold(s, True)
+        s.step(8)
+        with pytest.raises(fdtd.AefdtdError) as e:
+            READS[read](s)
+        assert e.value.status == TIMEOUT
+        withhold(s, False)
+        for call in (lambda s: s.step(1), READS["fields"], READS["flux"]):
+            with pytest.raises(fdtd.AefdtdError) as e:
+                call(s)
+            assert e.value.status == TIMEOUT
+        s.reset()
+        s.step(40)
+        assert np.array_equal(s.fields(), want)
+
+
+def test_a_reset_leaves_no_report_of_the_run_before():
+    scene = SCENES["cell"](precision=A.FP64)
+    want = run(scene, True, (40,))["fields"]
+    with fdtd.build_simulation(scene) as s:
+        withhold(s, True)
+        s.step(8)
+        s.reset()   # without a synchronising call before
+        withhold(s, False)
+        s.step(40)
+        s.synchronize()
+        assert np.array_equal(s.fields(), want)
