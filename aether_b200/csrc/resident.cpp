@@ -311,6 +311,7 @@ void aefdtd_sim::build_resident() {
     }
     if (cy.empty()) return;
     const int run = kernel.run;
+    AE_CUDA(fp64 ? prepare_resident_f64(run, (int)limit) : prepare_resident_f32(run, (int)limit));
     const int nb = (int)cy.size() - 1, ns = (int)cz.size() - 1;
     std::vector<ResBlock> B(size_t(nb) * ns);
     auto at = [&](int s, int b) -> ResBlock & { return B[size_t((s + ns) % ns) * nb + (b + nb) % nb]; };

@@ -1104,12 +1104,25 @@ __global__ void __launch_bounds__(NT, 1) resident_steps(const __grid_constant__ 
     if (B.nzp > 0) res_psi<T, L, NT, Tight, true>(A, B, s, i, J);
 }
 
-template <typename T, int L, int NT, bool Tight = false> cudaError_t launch_resident_run(const ResArgs<T> &A, int grid, int smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(resident_steps<T, L, NT, Tight>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+template <typename T> struct ResEntry {
+    void (*kernel)(const ResArgs<T>) = nullptr;
+    int threads = 0;
+};
+template <typename T, int L, int NT, bool Tight = false> ResEntry<T> resident_entry() { return {resident_steps<T, L, NT, Tight>, NT}; }
+
+// The attribute belongs to the kernel, not to a simulation: threads that step
+// simulations with different plans all set the same value, the device's limit.
+template <typename T> cudaError_t prepare_resident_entry(const ResEntry<T> &k, int most) {
+    if (!k.kernel) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
+template <typename T>
+cudaError_t launch_resident_entry(const ResEntry<T> &k, const ResArgs<T> &A, int grid, int smem, cudaStream_t st) {
+    if (!k.kernel) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NT);
+    cfg.blockDim = dim3(k.threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -1117,7 +1130,7 @@ template <typename T, int L, int NT, bool Tight = false> cudaError_t launch_resi
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, resident_steps<T, L, NT, Tight>, A);
+    return cudaLaunchKernelEx(&cfg, k.kernel, A);
 }
 
 }  // namespace aefdtd

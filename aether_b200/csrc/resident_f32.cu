@@ -2,18 +2,23 @@
 #include "resident.cuh"
 
 namespace aefdtd {
-cudaError_t launch_resident(const ResArgs<float> &A, int run, int grid, int smem, cudaStream_t s) {
+// The kernel with `run` planes per thread.
+static ResEntry<float> entry(int run) {
     switch (run) {
-        case 2: return launch_resident_run<float, 2, 512>(A, grid, smem, s);
-        case 4: return launch_resident_run<float, 4, 512>(A, grid, smem, s);
-        case 8: return launch_resident_run<float, 8, 384>(A, grid, smem, s);
-        case 12: return launch_resident_run<float, 12, 256>(A, grid, smem, s);
-        case 16: return launch_resident_run<float, 16, 256>(A, grid, smem, s);
-        case 20: return launch_resident_run<float, 20, 256>(A, grid, smem, s);
-        case 24: return launch_resident_run<float, 24, 256>(A, grid, smem, s);
-        case 25: return launch_resident_run<float, 25, 256, true>(A, grid, smem, s);
-        case 28: return launch_resident_run<float, 28, 256, true>(A, grid, smem, s);
-        default: return cudaErrorInvalidValue;
+        case 2: return resident_entry<float, 2, 512>();
+        case 4: return resident_entry<float, 4, 512>();
+        case 8: return resident_entry<float, 8, 384>();
+        case 12: return resident_entry<float, 12, 256>();
+        case 16: return resident_entry<float, 16, 256>();
+        case 20: return resident_entry<float, 20, 256>();
+        case 24: return resident_entry<float, 24, 256>();
+        case 25: return resident_entry<float, 25, 256, true>();
+        case 28: return resident_entry<float, 28, 256, true>();
+        default: return {};
     }
 }
+cudaError_t launch_resident(const ResArgs<float> &A, int run, int grid, int smem, cudaStream_t s) {
+    return launch_resident_entry(entry(run), A, grid, smem, s);
+}
+cudaError_t prepare_resident_f32(int run, int most) { return prepare_resident_entry(entry(run), most); }
 }  // namespace aefdtd

@@ -1,5 +1,7 @@
 """Resident time steps (resident.cuh) beside the normal run: a wait that runs
-out and how it is reported."""
+out and how it is reported, and several threads with a simulation each."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -54,3 +56,32 @@ def test_a_reset_leaves_no_report_of_the_run_before():
         s.step(40)
         s.synchronize()
         assert np.array_equal(s.fields(), want)
+
+
+def test_threads_with_plans_of_different_sizes():
+    """One owning thread per handle: launches of simulations whose plans take
+    the same kernel with different amounts of shared memory do not disturb
+    each other."""
+    names = ["gold_sphere", "slab_tm", "slab_te", "debye_lorentz_sphere"]
+    want = {n: run(SCENES[n](precision=A.FP64), True, (64,) * 6)["fields"] for n in names}
+    got, start = {}, threading.Barrier(len(names))
+
+    def work(name):
+        try:
+            with fdtd.build_simulation(SCENES[name](precision=A.FP64)) as s:
+                start.wait(60)
+                for _ in range(6):
+                    for _ in range(16):   # short calls: many launches
+                        s.step(4)
+                got[name] = s.fields()
+        except Exception as e:   # kept for the assertion below
+            got[name] = e
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in names]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for n in names:
+        assert isinstance(got[n], np.ndarray), got[n]
+        assert np.array_equal(got[n], want[n])
