@@ -402,7 +402,7 @@ void aefdtd_sim::build_resident() {
     // steps per launch: the sensor record within 8 MiB (64 MiB with DFT
     // planes), at least four steps, at most a segment
     const size_t room = size_t(sensors.empty() ? 8 : 64) << 20;
-    res.cap = res.rec ? (int)std::clamp<size_t>(room / (res.rec * es), 4, seg_len) : seg_len;
+    res.cap = res.rec ? (int)std::min<size_t>(seg_len, std::max<size_t>(4, room / (res.rec * es))) : seg_len;
     std::vector<char> host;
     auto put = [&](const void *p, size_t n) {
         const size_t o = host.size();

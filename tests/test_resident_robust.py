@@ -1,5 +1,6 @@
 """Resident time steps (resident.cuh) beside the normal run: a wait that runs
-out and how it is reported, and several threads with a simulation each."""
+out and how it is reported, several threads with a simulation each, and DFT
+blocks (so segments) of a few steps."""
 import threading
 
 import numpy as np
@@ -85,3 +86,19 @@ def test_threads_with_plans_of_different_sizes():
     for n in names:
         assert isinstance(got[n], np.ndarray), got[n]
         assert np.array_equal(got[n], want[n])
+
+
+@pytest.mark.parametrize("sensors", [True, False])
+@pytest.mark.parametrize("block", [1, 2, 3, 5])
+def test_segments_of_a_few_steps(block, sensors):
+    """A launch carries at most a segment (dft_block steps), however few."""
+    scene = SCENES["cell"](precision=A.FP64)
+    scene.grid.dft_block = block
+    if not sensors:
+        scene.sensors = []
+    a, b = run(scene, True, (1, 17, 4)), run(scene, False, (1, 17, 4))
+    for key in ("fields", "sums"):
+        assert np.array_equal(a[key], b[key])
+    for x, y in zip(a["dft"] + a["flux"], b["dft"] + b["flux"]):
+        assert np.array_equal(x, y)
+    assert len(a["flux"]) == len(scene.sensors)
