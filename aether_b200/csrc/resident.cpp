@@ -38,14 +38,23 @@ size_t up16(size_t b) { return (b + 15) / 16 * 16; }
 }  // namespace
 }  // namespace aefdtd
 
-// Whether the next steps can run resident: the drivers and sensors that the
+// Whether the next n steps can run resident: the drivers and sensors that the
 // resident kernel records sites for, ids of one byte, and a plan that fits.
 // The knobs that pin other kernels (and timing runs, which time the split
 // groups) keep their path.
-bool aefdtd_sim::resident_ready() {
+bool aefdtd_sim::resident_ready(int n) {
     if (!use_resident || batch || obl || timing || cc_coeff > 0 || !fmaps.empty() || id_bytes != 1 ||
         sensors.size() > (size_t)kMaxGather || fused_eligible() || use_tma)
         return false;
+    // A call of one step pays for loading and storing the whole state. The split
+    // kernels give the same bits in FP64 and take over there past 10 MB of
+    // fields; us per call, resident / split, without and with two flux planes:
+    // 12 x 10 x 90 24.7 / 27.9 and 31.3 / 37.0, 70 x 58 x 50 30.6 / 26.4 and 35.0
+    // / 37.1, 48 x 48 x 128 32.9 / 28.1 and 41.7 / 34.7, 64 x 64 x 128 43.1 / 31.7
+    // and 52.2 / 38.2; at two steps 31.6 / 33.4 per step. FP32 kernels round
+    // differently, so FP32 keeps to one path however a run is cut into calls (64 x
+    // 64 x 250: 47.2 / 30.5 per call of one step, 27.8 / 27.9 per step at two).
+    if (fp64 && n == 1 && 48.0 * Nx * Ny * Nz > 10e6) return false;
     if (res_dirty) build_resident();
     return res.grid > 0;
 }
@@ -159,7 +168,17 @@ void aefdtd_sim::build_resident() {
         else if (p->type <= 3) region(p->x1, p->y1, p->z1, p->span1 + 1, 2, p->span2 + 1, true);
         else region(p->x1, p->y1, p->z1, p->span1 + 1, p->span2 + 1, 2, true);
     }
-    if (res.rec > (size_t(1) << 30)) return;
+    // Steps per launch: at most a segment, and the sensor record within 8 MiB, or
+    // within 64 with DFT planes and where 8 hold fewer than `least` steps. A
+    // launch of few steps does not pay for loading and storing the state and for
+    // its sensor launches; us per step of 64 steps, resident / split, where a
+    // segment has 4 and 8 steps: 64 x 64 x 128 FP64 with two flux planes 30.9 /
+    // 26.0 and 20.4 / 21.4, 64 x 64 x 250 FP32 31.7 / 25.0 and 18.7 / 20.0; without
+    // flux planes, at 2 and 4 steps: 26.4 / 23.2 and 18.0 / 20.0, 27.8 / 23.6 and
+    // 18.8 / 20.0.
+    const size_t least = sensors.empty() ? 4 : 8, bytes = res.rec * es, most = size_t(64) << 20;
+    res.cap = bytes ? (int)std::min<size_t>(seg_len, std::max(least, (sensors.empty() ? most / 8 : most) / bytes)) : seg_len;
+    if (res.cap < (int)least || bytes * res.cap > most) return;
     // sensor sites in a block: the cells of each region's box that fall in it, with wraps
     auto sites_in = [&](const ResBlock &x) {
         size_t n = 0;
@@ -399,10 +418,6 @@ void aefdtd_sim::build_resident() {
         taps.insert(taps.end(), part[n].begin(), part[n].end());
         sites.insert(sites.end(), site[n].begin(), site[n].end());
     }
-    // steps per launch: the sensor record within 8 MiB (64 MiB with DFT
-    // planes), at least four steps, at most a segment
-    const size_t room = size_t(sensors.empty() ? 8 : 64) << 20;
-    res.cap = res.rec ? (int)std::min<size_t>(seg_len, std::max<size_t>(4, room / (res.rec * es))) : seg_len;
     std::vector<char> host;
     auto put = [&](const void *p, size_t n) {
         const size_t o = host.size();

@@ -940,7 +940,7 @@ void aefdtd_sim::run_steps(int n) {
     if (!work_dirty && (wsE.tma || wsH.tma) && !tma_maps_current()) work_dirty = true;
     // a grid that fits the SMs' shared memory stays there (resident.cuh); the
     // split path's work lists wait until they are needed
-    const bool resident = resident_ready();
+    const bool resident = resident_ready(n);
     if (work_dirty && !resident) { build_work(); graphs_dirty = true; fwork_dirty = true; }
     const bool fused = !resident && fused_eligible();
     if (fused) {

@@ -414,7 +414,7 @@ struct aefdtd_sim {
     bool use_resident = true;        // AEFDTD_RESIDENT
     bool res_dirty = true;           // the map, a material, a source or a sensor changed
     ResidentPlan res;
-    bool resident_ready();
+    bool resident_ready(int n);
     void build_resident();
     template <typename T> void run_resident(int n);
     // staged interior half-steps (interior_tma.cuh): curl-only 64 x 8 tiles

@@ -9,6 +9,7 @@ import pytest
 from aether_b200 import _abi as A
 from aether_b200 import fdtd
 from test_resident import SCENES, WAIT_CYCLES, WITHHOLD, run
+from test_resident_long import FP32 as FP32_LONG, FP64 as FP64_LONG
 
 pytestmark = pytest.mark.gpu
 TIMEOUT = 3   # AEFDTD_TIMEOUT
@@ -102,3 +103,40 @@ def test_segments_of_a_few_steps(block, sensors):
     for x, y in zip(a["dft"] + a["flux"], b["dft"] + b["flux"]):
         assert np.array_equal(x, y)
     assert len(a["flux"]) == len(scene.sensors)
+
+
+def runs_resident(scene, chunks):
+    """Whether the run issues fewer launches than the split kernels do."""
+    counts = [run(scene, resident, chunks)["launches"] for resident in (True, False)]
+    assert counts[0] <= counts[1]
+    return counts[0] < counts[1]
+
+
+def test_few_steps_per_launch_run_on_the_split_kernels():
+    """A launch of few steps does not pay for loading and storing the state:
+    short DFT blocks and, in FP64, single steps of the larger grids take the
+    split kernels, which give the same bits."""
+    scene = FP64_LONG["slab"](precision=A.FP64)
+    assert runs_resident(scene, (64,)) and runs_resident(scene, (2,))
+    assert not runs_resident(scene, (1,) * 4)
+    assert runs_resident(SCENES["gold_sphere"](precision=A.FP64), (1,) * 4)
+    for block in (1, 4, 7, 8):
+        scene.grid.dft_block = block
+        assert runs_resident(scene, (64,)) == (block >= 8), block
+    scene.sensors = []
+    for block in (3, 4):
+        scene.grid.dft_block = block
+        assert runs_resident(scene, (64,)) == (block >= 4), block
+
+
+@pytest.mark.parametrize("name,precision", [("slab", A.FP64), ("sphere_odd", A.FP64), ("slab", A.FP32)])
+def test_single_steps_among_longer_calls(name, precision):
+    """However a run is cut into calls: the same fields and sums, bit for bit,
+    and the flux up to the regrouping of its block sums."""
+    scene = {A.FP64: FP64_LONG, A.FP32: FP32_LONG}[precision][name](precision=precision)
+    a, b = run(scene, True, (100,)), run(scene, True, (1, 60, 1, 1, 2, 34, 1))
+    assert np.abs(a["fields"]).max() > 0
+    for key in ("fields", "sums"):
+        assert np.array_equal(a[key], b[key])
+    for x, y in zip(a["flux"], b["flux"]):
+        assert np.linalg.norm(x - y) <= (1e-10 if precision == A.FP64 else 1e-6) * np.linalg.norm(x)
