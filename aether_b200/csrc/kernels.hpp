@@ -41,9 +41,10 @@ template <typename T, typename Tid> int persist_capacity(int ty);
 // planes per thread, one of kResKernels32 / kResKernels64
 cudaError_t launch_resident(const ResArgs<double> &A, int run, int grid, int smem, cudaStream_t s);
 cudaError_t launch_resident(const ResArgs<float> &A, int run, int grid, int smem, cudaStream_t s);
-// before the first launch: lets the kernel take up to `most` bytes of shared memory
-cudaError_t prepare_resident_f64(int run, int most);
-cudaError_t prepare_resident_f32(int run, int most);
+// before the first launch: lets the kernel take up to `most` bytes of shared
+// memory; per_sm: its CTAs of `smem` bytes that an SM holds
+cudaError_t prepare_resident_f64(int run, int most, int smem, int &per_sm);
+cudaError_t prepare_resident_f32(int run, int most, int smem, int &per_sm);
 #define AEFDTD_DECL_PERSIST(T, Tid)                                                                    \
     cudaError_t launch_persist(const PersistArgs<T, Tid> &p, int grid, int ty, cudaStream_t s);        \
     template <> int persist_capacity<T, Tid>(int ty);

@@ -83,6 +83,7 @@ bool aefdtd_sim::resident_ready(int n) {
 void aefdtd_sim::build_resident() {
     res_dirty = false;
     res.grid = 0;
+    res.mem.release(dev_bytes);
     int nsm = 0, optin = 0, coop = 0;
     AE_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
     AE_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
@@ -330,7 +331,6 @@ void aefdtd_sim::build_resident() {
     }
     if (cy.empty()) return;
     const int run = kernel.run;
-    AE_CUDA(fp64 ? prepare_resident_f64(run, (int)limit) : prepare_resident_f32(run, (int)limit));
     const int nb = (int)cy.size() - 1, ns = (int)cz.size() - 1;
     std::vector<ResBlock> B(size_t(nb) * ns);
     auto at = [&](int s, int b) -> ResBlock & { return B[size_t((s + ns) % ns) * nb + (b + nb) % nb]; };
@@ -362,6 +362,15 @@ void aefdtd_sim::build_resident() {
             x.put_hy = x.self_y ? -1 : yp.get_h;
             x.put_hz = x.self_z ? -1 : zp.get_h + 2 * Nx * zp.bz;
         }
+    // What the device refuses (blocks that are not all resident at once, memory
+    // for the plan) is no error: the split kernels run in what there is.
+    int per_sm = 0;
+    if ((fp64 ? prepare_resident_f64(run, (int)limit, (int)smem, per_sm)
+              : prepare_resident_f32(run, (int)limit, (int)smem, per_sm)) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (per_sm * nsm < nb * ns || res.refuse == 2) return;
     std::vector<int> yb(Ny), zb(Nz);   // owner band / slab
     for (int b = 0; b < nb; b++) for (int j = cy[b]; j < cy[b + 1]; j++) yb[j] = b;
     for (int s = 0; s < ns; s++) for (int k = cz[s]; k < cz[s + 1]; k++) zb[k] = s;
@@ -431,7 +440,14 @@ void aefdtd_sim::build_resident() {
     res.sites = put(sites.data(), sizeof(uint2) * sites.size());
     res.inbox = host.size();
     res.raw = (res.inbox + up16(size_t(words) * 2 * es) + 255) / 256 * 256;
-    res.mem.alloc(res.raw + res.rec * es * res.cap, dev_bytes);
+    const size_t need = res.raw + res.rec * es * res.cap;
+    if (res.refuse == 1 || cudaMalloc(&res.mem.p, need) != cudaSuccess) {
+        cudaGetLastError();
+        res.mem.p = nullptr;
+        return;
+    }
+    res.mem.n = need;
+    dev_bytes += need;
     AE_CUDA(cudaMemcpy(res.mem.p, host.data(), host.size(), cudaMemcpyHostToDevice));
     AE_CUDA(cudaMemsetAsync(res.at<char>(res.inbox), 0, res.raw - res.inbox, stream));
     res.seq = 0;
@@ -442,8 +458,9 @@ void aefdtd_sim::build_resident() {
 
 // n steps in chunks of at most res.cap, each one cooperative launch and the
 // sensor launches over the sites it recorded; a chunk ends where a DFT sample
-// buffer fills, and the block is accumulated at once.
-template <typename T> void aefdtd_sim::run_resident(int n) {
+// buffer fills, and the block is accumulated at once. Returns the steps made:
+// fewer than n when a launch was refused, after which res.grid is 0.
+template <typename T> int aefdtd_sim::run_resident(int n) {
     for (auto *s : sensors) launch_pending<T>(*s, stream);
     std::vector<StepScalars> host(seg_len);
     int done = 0;
@@ -470,7 +487,16 @@ template <typename T> void aefdtd_sim::run_resident(int n) {
         A.abort = err.as<int>() + 1;
         A.wait_cycles = res.wait_cycles;
         A.withhold = res.withhold;
-        AE_CUDA(launch_resident(A, res.run, res.grid, res.smem, stream));
+        const cudaError_t refused =
+            res.refuse == 3 ? cudaErrorCooperativeLaunchTooLarge : launch_resident(A, res.run, res.grid, res.smem, stream);
+        // fewer SMs for this process than the device has, or no memory for the kernel's stack
+        if (refused == cudaErrorCooperativeLaunchTooLarge || refused == cudaErrorLaunchOutOfResources ||
+            refused == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            res.release(dev_bytes);
+            return done;
+        }
+        AE_CUDA(refused);
         launches++;
         int reg = 0;
         if (normal) {
@@ -507,6 +533,7 @@ template <typename T> void aefdtd_sim::run_resident(int n) {
         done += L;
     }
     AE_CUDA(cudaGetLastError());
+    return done;
 }
-template void aefdtd_sim::run_resident<double>(int);
-template void aefdtd_sim::run_resident<float>(int);
+template int aefdtd_sim::run_resident<double>(int);
+template int aefdtd_sim::run_resident<float>(int);

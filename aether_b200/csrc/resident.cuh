@@ -1112,9 +1112,11 @@ template <typename T, int L, int NT, bool Tight = false> ResEntry<T> resident_en
 
 // The attribute belongs to the kernel, not to a simulation: threads that step
 // simulations with different plans all set the same value, the device's limit.
-template <typename T> cudaError_t prepare_resident_entry(const ResEntry<T> &k, int most) {
+template <typename T> cudaError_t prepare_resident_entry(const ResEntry<T> &k, int most, int smem, int &per_sm) {
+    per_sm = 0;
     if (!k.kernel) return cudaErrorInvalidValue;
-    return cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const cudaError_t e = cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.kernel, k.threads, smem);
 }
 
 template <typename T>

@@ -20,5 +20,7 @@ static ResEntry<double> entry(int run) {
 cudaError_t launch_resident(const ResArgs<double> &A, int run, int grid, int smem, cudaStream_t s) {
     return launch_resident_entry(entry(run), A, grid, smem, s);
 }
-cudaError_t prepare_resident_f64(int run, int most) { return prepare_resident_entry(entry(run), most); }
+cudaError_t prepare_resident_f64(int run, int most, int smem, int &per_sm) {
+    return prepare_resident_entry(entry(run), most, smem, per_sm);
+}
 }  // namespace aefdtd

@@ -963,7 +963,8 @@ void aefdtd_sim::run_steps(int n) {
         drop_graphs();
     }
     if (resident) {
-        run_resident<T>(n);
+        const int done = run_resident<T>(n);
+        if (done < n) run_steps<T, Tid>(n - done);   // refused: the split kernels take the rest
         return;
     }
     if (obl && tstep + n > obl->cap) {
@@ -2447,6 +2448,10 @@ aefdtd_status aefdtd_test_hook(aefdtd_sim *s, int32_t what, int64_t value) {
             s->res.wait_cycles = value;
         } else if (what == AEFDTD_TEST_RESIDENT_WITHHOLD) {
             s->res.withhold = value ? 1 : 0;
+        } else if (what == AEFDTD_TEST_RESIDENT_REFUSE) {
+            if (value < 0 || value > 3) fail(AEFDTD_BAD_ARG, "refusals are 0 to 3");
+            s->res.refuse = (int)value;
+            s->res_dirty = true;
         } else {
             fail(AEFDTD_BAD_ARG, "unknown test hook");
         }

@@ -204,6 +204,7 @@ struct ResidentPlan {
     unsigned seq = 0;              // half-steps numbered so far on the inboxes
     long long wait_cycles = 1LL << 31;   // bound of each wait, and the test hook (aefdtd_test_hook)
     int withhold = 0;
+    int refuse = 0;                // test hook
     // one allocation: blocks, dispersive cells, taps, sites, inboxes, records
     DBuf mem;
     size_t disp = 0, taps = 0, sites = 0, inbox = 0, raw = 0;   // their byte offsets
@@ -416,7 +417,7 @@ struct aefdtd_sim {
     ResidentPlan res;
     bool resident_ready(int n);
     void build_resident();
-    template <typename T> void run_resident(int n);
+    template <typename T> int run_resident(int n);
     // staged interior half-steps (interior_tma.cuh): curl-only 64 x 8 tiles
     // whose planes arrive through tensor copies. Not for batch members (their
     // merged lists take every interior item) or the oblique driver (whose

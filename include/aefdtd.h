@@ -465,6 +465,10 @@ aefdtd_status aefdtd_probe_copy_bandwidth(int32_t device, size_t bytes, int32_t 
  * step. */
 #define AEFDTD_TEST_RESIDENT_WAIT_CYCLES 7
 #define AEFDTD_TEST_RESIDENT_WITHHOLD 8
+/* Where a resident plan is refused, as if by the device: 1 its memory, 2 its
+ * blocks by the occupancy query, 3 its launch; 0 for no refusal. The simulation
+ * then takes the split half-steps until its set-up changes. */
+#define AEFDTD_TEST_RESIDENT_REFUSE 9
 aefdtd_status aefdtd_test_hook(aefdtd_sim *sim, int32_t what, int64_t value);
 
 /* ---- batches: many simulations advanced together ----------------------

@@ -1,6 +1,6 @@
 """Resident time steps (resident.cuh) beside the normal run: a wait that runs
-out and how it is reported, several threads with a simulation each, and DFT
-blocks (so segments) of a few steps."""
+out and how it is reported, several threads with a simulation each, DFT blocks
+(so segments) of a few steps, and a device that refuses the plan."""
 import threading
 
 import numpy as np
@@ -21,6 +21,7 @@ def withhold(s, on):
     assert s._lib.aefdtd_test_hook(s._h, WITHHOLD, int(on)) == 0
 
 
+REFUSE = 9    # AEFDTD_TEST_RESIDENT_REFUSE
 READS = {"fields": lambda s: s.fields(), "sums": lambda s: s.plane_sums(), "spectra": lambda s: s.normal_spectra(),
          "flux": lambda s: s.sensor_flux(1), "dft": lambda s: s.sensor_dft(0), "synchronize": lambda s: s.synchronize()}
 
@@ -140,3 +141,29 @@ def test_single_steps_among_longer_calls(name, precision):
         assert np.array_equal(a[key], b[key])
     for x, y in zip(a["flux"], b["flux"]):
         assert np.linalg.norm(x - y) <= (1e-10 if precision == A.FP64 else 1e-6) * np.linalg.norm(x)
+
+
+@pytest.mark.parametrize("name", ["gold_sphere", "box"])
+@pytest.mark.parametrize("where", [1, 2, 3])
+def test_a_refused_plan_falls_back_to_the_split_kernels(where, name):
+    """No memory for the plan, blocks that do not fit at once, a refused launch
+    (also after resident steps): the run goes on as if there were no resident
+    path, and takes it again when the refusal and the plan are gone."""
+    scene = SCENES[name](precision=A.FP64)
+    want = run(scene, False, (40, 30, 30))
+    with fdtd.build_simulation(scene) as s:
+        assert s._lib.aefdtd_test_hook(s._h, REFUSE, where) == 0
+        s.step(40)
+        n = s.launch_count()
+        assert n >= 3 * 40   # launches: E, H and their sensors or boundaries each step
+        assert s._lib.aefdtd_test_hook(s._h, REFUSE, 0) == 0
+        s.step(30)
+        assert s.launch_count() < n + 60
+        assert s._lib.aefdtd_test_hook(s._h, REFUSE, where) == 0
+        s.step(30)
+        assert np.array_equal(s.fields(), want["fields"])
+        for i in range(len(s.sensor_nl)):
+            if i < len(scene.sensors):
+                assert np.array_equal(s.sensor_flux(i), want["flux"][i])
+        if "sums" in want:
+            assert np.array_equal(s.plane_sums(), want["sums"])
