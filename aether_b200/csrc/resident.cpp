@@ -216,13 +216,15 @@ void aefdtd_sim::build_resident() {
         x.feat_e = kernel_feat(fe);
         x.feat_h = kernel_feat(f);
     };
-    // psi slots of a block's runs: the planes from a run's first z-CPML plane to its last
+    // psi slots of a block's runs: a run's z-CPML planes, of one end of the axis
+    // (-1: a run reaches both, which its record has no room for)
     auto slots = [&](const ResBlock &x, int run) {
         int n = 0;
         for (int r = 0; pz && r < x.nseg; r++) {
             const int k = x.k0 + r * run, e = std::min(k + run, x.k0 + x.bz);
-            const bool low = k < pml[4], high = e > Nz - pml[5];
-            if (low || high) n = std::max(n, (high ? e : std::min(e, pml[4])) - (low ? k : std::max(k, Nz - pml[5])));
+            const int low = std::min(e, pml[4]) - k, high = e - std::max(k, Nz - pml[5]);
+            if (low > 0 && high > 0) return -1;
+            n = std::max({n, low, high});
         }
         return n;
     };
@@ -317,7 +319,7 @@ void aefdtd_sim::build_resident() {
                         ResBlock &y = x[m];
                         y.nseg = (y.bz + K.run - 1) / K.run;
                         worst = std::max(worst, waits + cost(y, K));
-                        better = y.disp_n < kResNoRank && worst < best && !(K.tight && ((y.feat_e | y.feat_h) & kXY));
+                        better = y.disp_n < kResNoRank && worst < best && slots(y, K.run) >= 0 && !(K.tight && ((y.feat_e | y.feat_h) & kXY));
                     }
                     for (size_t m = 0; m < x.size() && better; m++) better = layout(x[m], K) <= limit;
                     if (!better) continue;

@@ -98,8 +98,7 @@ __device__ __forceinline__ Coef4<double> coef4(const MatCoef<double> *c) {
 
 // Shared memory of a CTA, in values of T from the start: E [3][L][threads],
 // H [3][L][threads] (Tight: in the same place, see resident_steps), z-CPML psi
-// [E 0, E 1, H 0, H 1][npsi][threads], a slot for each plane from a run's first
-// CPML plane to its last.
+// [E 0, E 1, H 0, H 1][npsi][threads], a slot for each CPML plane of a run.
 extern __shared__ __align__(16) unsigned char res_sm[];
 template <typename T, int L, int NT> __device__ __forceinline__ T *res_e(int c) { return reinterpret_cast<T *>(res_sm) + c * L * NT; }
 template <typename T, int L, int NT, bool Tight> __device__ __forceinline__ T *res_h(int c) {
@@ -120,9 +119,10 @@ template <typename T, int L> struct ResThread {
     T e0[L], e1[L], e2[L], h0[L], h1[L], h2[L];
     int K;                              // first plane
 };
-// z-CPML values of one of the block's planes for E and for H. Outside a side's
-// range b keeps psi (which is zero there) and c adds nothing, so the updates
-// need no branch; planes without a slot read zero.
+// z-CPML values of one of the block's planes for E and for H. The updates need no
+// branch on the range (taking one cost a 60 x 60 x 200 FP32 cell 9 %): outside it
+// psi is zero, chosen after the recursion, as its c = 0 would add 0 * inf, a NaN
+// where the split kernels have none.
 template <typename T> struct alignas(16) ResZ { T ik, b, c, pad; };
 // Material id of a thread's run plane k: a word of shared memory per four planes.
 template <int NT> __device__ __forceinline__ int res_id(const ResBlock &B, int k) {
@@ -295,11 +295,11 @@ __device__ __forceinline__ void res_cell_h(const StepArgs<T, uint8_t> &a, const 
 template <typename T> struct ResRow {
     const T *row, *plane;
     int sj, dj, dz, x;
-    int nk, lo, np;       // the run's planes, its first z-CPML plane and the planes to its last
+    int nk, lo, from, np; // the run's planes, its first z-CPML plane (of either half-step), this half-step's first and how many
     int face_y, face_z;   // places in the halo, -1 for none
 };
 // The record: two words per half-step and thread, computed once per launch.
-// p: element | halo << 16 | x << 17; z: element | halo << 16 | nk << 17 | lo << 22 | np << 27.
+// p: element | halo << 16 | x << 17 | lo << 26; z: element | halo << 16 | nk << 17 | from << 22 | np << 27.
 template <int L> struct ResPack {
     static_assert(L < 32, "a run's planes are packed in five bits");
     static constexpr unsigned kHalo = 1u << 16;   // above any element of 227 KB
@@ -323,11 +323,15 @@ __device__ __forceinline__ uint2 res_pack(const StepArgs<T, uint8_t> &a, const R
         z = (halo + 2 * nx * B.bz + col) | ResPack<L>::kHalo;
     }
     const int x = !live ? t : HALF ? (i < nx - 1 ? t + 1 : t - (nx - 1)) : (i ? t - 1 : t + nx - 1);
-    // planes of the run in [0, pml_zm) and [Nz - pml_zp, Nz)
+    // planes of the run in the range of E, [1, pml_zm) and [Nz - pml_zp + 1, Nz), or
+    // of H, [0, pml_zm) and [Nz - pml_zp, Nz - 1) (fdtd_pml.cpp:547,559,775,784);
+    // no run holds planes of both ends (resident.cpp)
     const int K = B.k0 + kb, nk = live ? min(L, B.bz - kb) : 0;
     const int low = a.pz ? max(0, min(nk, a.pml_zm - K)) : 0, high = a.pz ? min(nk, max(0, a.Nz - a.pml_zp - K)) : nk;
-    const int lo = low > 0 ? 0 : high, np = high < nk ? nk - lo : low;
-    return make_uint2(p | x << 17, z | nk << 17 | lo << 22 | unsigned(np) << 27);
+    const int lo = low > 0 ? 0 : high;
+    const int from = low > 0 ? (!HALF && K == 0) : min(nk, high + (!HALF && high < nk && K + high == a.Nz - a.pml_zp));
+    const int to = low > 0 ? low : HALF && nk > high && K + nk == a.Nz ? nk - 1 : nk;
+    return make_uint2(p | x << 17 | unsigned(lo) << 26, z | nk << 17 | from << 22 | unsigned(to - from) << 27);
 }
 template <typename T> __device__ __forceinline__ const T *res_at(int element) { return reinterpret_cast<const T *>(res_sm) + element; }
 template <typename T, int L, int NT, int HALF> __device__ __forceinline__ ResRow<T> res_record(int nx, const ResBlock &B) {
@@ -340,9 +344,10 @@ template <typename T, int L, int NT, int HALF> __device__ __forceinline__ ResRow
     r.sj = hp ? nx : NT;
     r.dj = hp ? nx * B.bz : 2 * L * NT;
     r.dz = hz ? nx * B.by : L * NT;
-    r.x = w.x >> 17;
+    r.x = w.x >> 17 & 511;
     r.nk = w.y >> 17 & 31;
-    r.lo = w.y >> 22 & 31;
+    r.lo = w.x >> 26;
+    r.from = w.y >> 22 & 31;
     r.np = w.y >> 27;
     r.face_y = hp && r.nk > 0 ? p - halo : -1;
     r.face_z = hz && r.nk > 0 ? z - halo : -1;
@@ -361,6 +366,7 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
     const ResRow<T> next = res_record<T, L, NT, 0>(A.e.Nx, B);
     const T *row = next.row, *plane = next.plane;
     const int sj = next.sj, dj = next.dj, nk = next.nk, lo = next.lo;
+    const auto on = [&](int k) { return unsigned(k - next.from) < unsigned(next.np); };   // in the z-CPML range
     const MatCoef<T> *coef = reinterpret_cast<const MatCoef<T> *>(res_sm + B.o_coef);
     const ResZ<T> *zt = reinterpret_cast<const ResZ<T> *>(res_sm + B.o_z) + (s.K - B.k0);
     // the run's coefficients where it has one material
@@ -397,9 +403,8 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
             if constexpr ((F & kFDisp) != 0) rank[u] = reinterpret_cast<const uint16_t *>(res_sm + B.o_rank)[k * NT + threadIdx.x];
             if constexpr ((F & kFPmlZ) != 0) {
                 z[u] = zt[k];
-                const bool slot = unsigned(k - lo) < unsigned(next.np);
-                p0[u] = slot ? pz0[k * NT] : T(0);
-                p1[u] = slot ? pz1[k * NT] : T(0);
+                p0[u] = on(k) ? pz0[k * NT] : T(0);
+                p1[u] = on(k) ? pz1[k * NT] : T(0);
             }
         }
         if constexpr ((F & kFDisp) != 0 && kBatchSums) {
@@ -446,9 +451,9 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
                 }
             if constexpr ((F & kFPmlZ) != 0) {
                 const T C4 = Mixed ? coef[res_id<NT>(B, k)].C4 : C41;
-                p0[u] = cpml_rec(z[u].b, p0[u], z[u].c, dHy_z);
+                p0[u] = on(k) ? cpml_rec(z[u].b, p0[u], z[u].c, dHy_z) : T(0);
                 nex -= C4 * p0[u];
-                p1[u] = cpml_rec(z[u].b, p1[u], z[u].c, dHx_z);
+                p1[u] = on(k) ? cpml_rec(z[u].b, p1[u], z[u].c, dHx_z) : T(0);
                 ney += C4 * p1[u];
                 nex = k == kpec ? T(0) : nex;
                 ney = k == kpec ? T(0) : ney;
@@ -464,7 +469,7 @@ __device__ __forceinline__ void res_run_e(const ResArgs<T> &A, const ResBlock &B
         if constexpr ((F & kFPmlZ) != 0) {
 #pragma unroll
             for (int u = 0; u < C; ++u)
-                if (k0 + u < L && unsigned(k0 + u - lo) < unsigned(next.np)) {
+                if (k0 + u < L && on(k0 + u)) {
                     pz0[(k0 + u) * NT] = p0[u];
                     pz1[(k0 + u) * NT] = p1[u];
                 }
@@ -477,6 +482,7 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
     const ResRow<T> next = res_record<T, L, NT, 1>(A.e.Nx, B);
     const T *row = next.row, *plane = next.plane;
     const int sj = next.sj, dj = next.dj, nk = next.nk, lo = next.lo;
+    const auto on = [&](int k) { return unsigned(k - next.from) < unsigned(next.np); };   // in the z-CPML range
     const ResZ<T> *zt = reinterpret_cast<const ResZ<T> *>(res_sm + B.o_z) + B.bz + L + (s.K - B.k0);
     const int kin = A.h.kinj - s.K, kpec = A.h.pz ? A.h.Nz - 1 - s.K : -1;
     T injA = 0, injB = 0;
@@ -503,9 +509,8 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
             x2[u] = res_e<T, L, NT>(2)[k * NT + next.x];
             if constexpr ((F & kFPmlZ) != 0) {
                 z[u] = zt[k];
-                const bool slot = unsigned(k - lo) < unsigned(next.np);
-                p0[u] = slot ? pz0[k * NT] : T(0);
-                p1[u] = slot ? pz1[k * NT] : T(0);
+                p0[u] = on(k) ? pz0[k * NT] : T(0);
+                p1[u] = on(k) ? pz1[k * NT] : T(0);
             }
         }
 #pragma unroll
@@ -522,9 +527,9 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
             T nhy = s.h1[k] + (ax * dEz_x - az * dEx_z);
             const T nhz = s.h2[k] + (ay * dEx_y - ax * dEy_x);
             if constexpr ((F & kFPmlZ) != 0) {
-                p0[u] = cpml_rec(z[u].b, p0[u], z[u].c, dEy_z);
+                p0[u] = on(k) ? cpml_rec(z[u].b, p0[u], z[u].c, dEy_z) : T(0);
                 nhx += dtm * p0[u];
-                p1[u] = cpml_rec(z[u].b, p1[u], z[u].c, dEx_z);
+                p1[u] = on(k) ? cpml_rec(z[u].b, p1[u], z[u].c, dEx_z) : T(0);
                 nhy -= dtm * p1[u];
                 nhx = k == kpec ? T(0) : nhx;
                 nhy = k == kpec ? T(0) : nhy;
@@ -538,7 +543,7 @@ __device__ __forceinline__ void res_run_h(const ResArgs<T> &A, const ResBlock &B
         if constexpr ((F & kFPmlZ) != 0) {
 #pragma unroll
             for (int u = 0; u < C; ++u)
-                if (k0 + u < L && unsigned(k0 + u - lo) < unsigned(next.np)) {
+                if (k0 + u < L && on(k0 + u)) {
                     pz0[(k0 + u) * NT] = p0[u];
                     pz1[(k0 + u) * NT] = p1[u];
                 }
@@ -909,18 +914,16 @@ __device__ __forceinline__ void res_psi(const ResArgs<T> &A, const ResBlock &B, 
     const StepArgs<T, uint8_t> &a = A.e;
     T *const g[4] = {A.e.psi_z0, A.e.psi_z1, A.h.psi_z0, A.h.psi_z1};
 #pragma unroll 1
-    for (int n = 0; n < at.np; ++n) {
+    for (int n = 0; at.lo + n < at.nk; ++n) {
         const int K = s.K + at.lo + n;
-        const int zn = K < a.pml_zm ? K : K >= a.Nz - a.pml_zp ? K - (a.Nz - a.pml_zp) + a.pml_zm : -1;
+        if (K >= a.pml_zm && K < a.Nz - a.pml_zp) break;
+        const int zn = K < a.pml_zm ? K : K - (a.Nz - a.pml_zp) + a.pml_zm;
         const long long o = i + (long long)J * a.Nx + zn * a.NxNy;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             T *p = res_pz<T, L, NT, Tight>(B.npsi, q) + n * NT;
-            if constexpr (Store) {
-                if (zn >= 0) g[q][o] = *p;
-            } else {
-                *p = zn >= 0 ? g[q][o] : T(0);
-            }
+            if constexpr (Store) g[q][o] = *p;
+            else *p = g[q][o];
         }
     }
 }

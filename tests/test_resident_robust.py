@@ -1,6 +1,7 @@
 """Resident time steps (resident.cuh) beside the normal run: a wait that runs
 out and how it is reported, several threads with a simulation each, DFT blocks
-(so segments) of a few steps, and a device that refuses the plan."""
+(so segments) of a few steps, a device that refuses the plan, and fields with
+infinities."""
 import threading
 
 import numpy as np
@@ -167,3 +168,34 @@ def test_a_refused_plan_falls_back_to_the_split_kernels(where, name):
                 assert np.array_equal(s.sensor_flux(i), want["flux"][i])
         if "sums" in want:
             assert np.array_equal(s.plane_sums(), want["sums"])
+
+
+@pytest.mark.parametrize("precision", [A.FP64, A.FP32])
+@pytest.mark.parametrize("name", ["slab_tm", "gold_sphere", "poles_in_cpml", "thin_column", "custom_box"])
+def test_infinities_and_nans_spread_as_in_the_split_kernels(name, precision, monkeypatch):
+    """Infinite and NaN values in and beside the CPML, at the faces of blocks
+    and in the interior: the same cells are finite, infinite and NaN after
+    three steps (the shortest run that sees both updates of both)."""
+    scene = SCENES[name](precision=precision)
+    nx, ny, nz = scene.total_dims()
+    rng = np.random.default_rng(8)
+    start = rng.standard_normal((6, nz, ny, nx))
+    for c in range(6):
+        for v in (np.inf, -np.inf, np.nan):
+            for k in rng.integers(0, nz, 3):
+                start[c, k, rng.integers(0, ny), rng.integers(0, nx)] = v
+        start[c, 0, 0, 0] = start[c, nz - 1, ny - 1, nx - 1] = np.inf
+    got = []
+    for resident in ("1", "0"):
+        monkeypatch.setenv("AEFDTD_RESIDENT", resident)
+        with fdtd.build_simulation(scene) as s:
+            for c in range(6):
+                s.set_field(c, start[c])
+            s.step(3)
+            got.append((s.fields(), s.launch_count()))
+    (a, na), (b, nb) = got
+    assert na < nb
+    assert np.array_equal(np.isnan(a), np.isnan(b)) and np.isnan(b).any()
+    assert np.array_equal(np.isinf(a), np.isinf(b)) and np.isinf(b).any()
+    if precision == A.FP64:
+        assert np.array_equal(a, b, equal_nan=True)
