@@ -74,8 +74,12 @@ struct Ctx {
 __device__ __forceinline__ double vmod(double v, double m, const VoxArgs &a) {
     // modulus (src/common/mathUT.h:606-612), with a bound on the walk
     int n = 0;
-    while (v < 0) { v += m; if (++n > kMaxMarch) { atomicExch(a.err, 1); return 0; } }
-    while (v >= m) { v -= m; if (++n > kMaxMarch) { atomicExch(a.err, 1); return 0; } }
+    for (; v < 0 && n <= kMaxMarch; ++n) v += m;
+    for (; v >= m && n <= kMaxMarch; ++n) v -= m;
+    if (n > kMaxMarch) {
+        atomicExch(a.err, 1);
+        v = 0;
+    }
     return v;
 }
 
@@ -321,7 +325,7 @@ __device__ __noinline__ int struct_index(const VoxArgs &a, double x, double y, d
 // corners. A CTA
 // now tags a tile of corners: it first lists, in that order, the images whose
 // primitive can contain a corner of the tile, up to the first that contains all
-// of it, and its corners test only those: 0.27 ms.
+// of it, and its corners test only those: 0.20 ms.
 //
 // What may be left out. With lo and hi the smallest and largest coordinate of
 // the tile's corners per axis, rounding is monotone, so a primitive's own
@@ -336,26 +340,29 @@ constexpr int kTilePoints = 1024, kTileThreads = 128, kMaxImages = 256 * 27;
 struct TileBox { double lo[3], hi[3]; };
 
 // 0: no corner of the box is in the primitive; 2: all are; 1: some may be.
-// A call, and the layer's axis chosen by selects: inlined, and with the axis as
-// an index into the box, nvcc 12.9 gave layers wrong results in warps that hold
-// other kinds too (tests/test_voxel_tiles.py).
-__device__ __noinline__ int tile_hits(const VoxOp &o, const TileBox &b) {
+//
+// No return or break out of a loop here and in vmod: votes and barriers follow.
+// With returns from the loops, inlined, nvcc 12.9 left the warp diverged behind
+// them (clock64 showed lanes of one warp at the vote 830 cycles apart), each part
+// voted and passed the barrier by itself, and lists lost images
+// (tests/test_voxel_tiles.py). As written the lanes arrive together.
+__device__ __forceinline__ int tile_hits(const VoxOp &o, const TileBox &b) {
     const double *p = o.p;
-    const auto outside = [&](int t, double from, double to) { return b.hi[t] < from || b.lo[t] > to; };
+    bool out = false, all = false;
     switch (o.kind) {
-        case AEFDTD_OP_BLOCK: {
-            bool all = true;
+        case AEFDTD_OP_BLOCK:
+            all = true;
             for (int t = 0; t < 3; t++) {
-                if (b.hi[t] < p[2 * t] || b.lo[t] >= p[2 * t + 1]) return 0;
-                all = all && b.lo[t] >= p[2 * t] && b.hi[t] < p[2 * t + 1];
+                out |= (b.hi[t] < p[2 * t]) | (b.lo[t] >= p[2 * t + 1]);
+                all &= (b.lo[t] >= p[2 * t]) & (b.hi[t] < p[2 * t + 1]);
             }
-            return all ? 2 : 1;
-        }
+            break;
         case AEFDTD_OP_LAYER: {
             const int t = (int)p[0];
             const double lo = t == 0 ? b.lo[0] : t == 1 ? b.lo[1] : b.lo[2], hi = t == 0 ? b.hi[0] : t == 1 ? b.hi[1] : b.hi[2];
-            if (hi < p[1] || lo >= p[2]) return 0;
-            return lo >= p[1] && hi < p[2] ? 2 : 1;
+            out = (hi < p[1]) | (lo >= p[2]);
+            all = (lo >= p[1]) & (hi < p[2]);
+            break;
         }
         case AEFDTD_OP_SPHERE: {
             double d2 = 0;
@@ -363,29 +370,28 @@ __device__ __noinline__ int tile_hits(const VoxOp &o, const TileBox &b) {
                 const double d = b.hi[t] < p[t] ? p[t] - b.hi[t] : b.lo[t] > p[t] ? b.lo[t] - p[t] : 0.0;
                 d2 += d * d;
             }
-            return d2 > p[3] * p[3] * (1.0 + 1e-9) ? 0 : 1;
+            out = d2 > p[3] * p[3] * (1.0 + 1e-9);
+            break;
         }
         case AEFDTD_OP_CYLINDER:
         case AEFDTD_OP_CONE:
-            for (int t = 0; t < 3; t++)
-                if (outside(t, fmin(p[t], p[3 + t]) - p[6], fmax(p[t], p[3 + t]) + p[6])) return 0;
-            return 1;
+            for (int t = 0; t < 3; t++) out |= (b.hi[t] < fmin(p[t], p[3 + t]) - p[6]) | (b.lo[t] > fmax(p[t], p[3 + t]) + p[6]);
+            break;
         case AEFDTD_OP_ELLIPSOID:
-            for (int t = 0; t < 3; t++)
-                if (outside(t, p[t] - p[3 + t], p[t] + p[3 + t])) return 0;
-            return 1;
+            for (int t = 0; t < 3; t++) out |= (b.hi[t] < p[t] - p[3 + t]) | (b.lo[t] > p[t] + p[3 + t]);
+            break;
         case AEFDTD_OP_VECT_BLOCK:
         case AEFDTD_OP_VECT_TRI:
         case AEFDTD_OP_MESH:
-            for (int t = 0; t < 3; t++)
-                if (outside(t, o.vmin[t], o.vmax[t])) return 0;
-            return 1;
+            for (int t = 0; t < 3; t++) out |= (b.hi[t] < o.vmin[t]) | (b.lo[t] > o.vmax[t]);
+            break;
     }
-    return 1;
+    return out ? 0 : all ? 2 : 1;
 }
 
 // Tiles of tx x ty x tz corners (powers of two, tz * tx * ty = kTilePoints); a
-// thread's corners are one column of them or several.
+// thread's corners are one column of them or several. A CTA takes one tile: the
+// primitives' own tests, which leave from anywhere, are the last that it does.
 __global__ void __launch_bounds__(kTileThreads) voxelize_kernel(const __grid_constant__ VoxArgs a, int tx, int ty) {
     const int tz = kTilePoints / (tx * ty), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntx = (a.nx + tx - 1) / tx, nty = (a.ny + ty - 1) / ty, ntz = (a.nz + tz - 1) / tz;
@@ -395,94 +401,92 @@ __global__ void __launch_bounds__(kTileThreads) voxelize_kernel(const __grid_con
     __shared__ unsigned short list[kMaxImages];
     __shared__ int warp_n[kTileThreads / 32], stop, total;
     double *const X[3] = {pos, pos + kTilePoints, pos + 2 * kTilePoints};
-    for (long long tile = blockIdx.x; tile < (long long)ntx * nty * ntz; tile += gridDim.x) {
-        const int o0[3] = {(int)(tile % ntx) * tx, (int)(tile / ntx % nty) * ty, (int)(tile / ((long long)ntx * nty)) * tz};
-        const int cnt[3] = {min(tx, a.nx - o0[0]), min(ty, a.ny - o0[1]), min(tz, a.nz - o0[2])};
-        __syncthreads();   // the tile before is done with pos, list and total
-        for (int t = 0; t < 3; t++) {
-            const double step = t == 0 ? a.dx : t == 1 ? a.dy : a.dz;
-            for (int n = tid; n < cnt[t]; n += kTileThreads) {
-                double v = (o0[t] + n) * step;
-                if (a.flip[t]) v = a.l[t] - v;
-                if (a.per[t]) v = vmod(v, a.l[t], a);
-                X[t][n] = v;
+    const long long tile = blockIdx.x;
+    const int o0[3] = {(int)(tile % ntx) * tx, (int)(tile / ntx % nty) * ty, (int)(tile / ((long long)ntx * nty)) * tz};
+    const int cnt[3] = {min(tx, a.nx - o0[0]), min(ty, a.ny - o0[1]), min(tz, a.nz - o0[2])};
+    for (int t = 0; t < 3; t++) {
+        const double step = t == 0 ? a.dx : t == 1 ? a.dy : a.dz;
+        for (int n = tid; n < cnt[t]; n += kTileThreads) {
+            double v = (o0[t] + n) * step;
+            if (a.flip[t]) v = a.l[t] - v;
+            if (a.per[t]) v = vmod(v, a.l[t], a);
+            X[t][n] = v;
+        }
+    }
+    if (tid == 0) {
+        total = 0;
+        stop = 0;
+    }
+    __syncthreads();
+    if (warp < 3) {   // a warp per axis
+        // a NaN coordinate makes the box NaN, which keeps every image
+        double lo = X[warp][0], hi = lo;
+        for (int n = lane; n < cnt[warp]; n += 32) {
+            const double v = X[warp][n];
+            lo = v < lo || v != v ? v : lo;
+            hi = v > hi || v != v ? v : hi;
+        }
+        for (int d = 16; d; d >>= 1) {
+            const double l2 = __shfl_xor_sync(0xffffffffu, lo, d), h2 = __shfl_xor_sync(0xffffffffu, hi, d);
+            lo = l2 < lo || l2 != l2 ? l2 : lo;
+            hi = h2 > hi || h2 != h2 ? h2 : hi;
+        }
+        if (lane == 0) {
+            box.lo[warp] = lo;
+            box.hi[warp] = hi;
+        }
+    }
+    __syncthreads();
+    // the images in the order of struct_index: last operation first
+    for (int e0 = 0; e0 < a.nops * images && !stop; e0 += kTileThreads) {
+        const int e = e0 + tid, op = e / images, im = e - op * images;
+        int hit = 0;
+        if (op < a.nops) {
+            const int d[3] = {im / (nj * nk) - a.per[0], im / nk % nj - a.per[1], im % nk - a.per[2]};
+            TileBox b;
+            for (int t = 0; t < 3; t++) {
+                b.lo[t] = box.lo[t] + d[t] * a.l[t];
+                b.hi[t] = box.hi[t] + d[t] * a.l[t];
             }
+            hit = tile_hits(a.ops[a.nops - 1 - op], b);
         }
-        if (tid == 0) {
-            total = 0;
-            stop = 0;
-        }
+        // nothing below an image that contains the tile is reached
+        const unsigned some = __ballot_sync(0xffffffffu, hit != 0), all = __ballot_sync(0xffffffffu, hit == 2);
+        const unsigned keep = all ? some & ((2u << (__ffs(all) - 1)) - 1) : some;
+        if (lane == 0) warp_n[warp] = __popc(keep) | (all ? 1 << 16 : 0);
         __syncthreads();
-        if (warp < 3) {   // a warp per axis
-            // a NaN coordinate makes the box NaN, which keeps every image
-            double lo = X[warp][0], hi = lo;
-            for (int n = lane; n < cnt[warp]; n += 32) {
-                const double v = X[warp][n];
-                lo = v < lo || v != v ? v : lo;
-                hi = v > hi || v != v ? v : hi;
-            }
-            for (int d = 16; d; d >>= 1) {
-                const double l2 = __shfl_xor_sync(0xffffffffu, lo, d), h2 = __shfl_xor_sync(0xffffffffu, hi, d);
-                lo = l2 < lo || l2 != l2 ? l2 : lo;
-                hi = h2 > hi || h2 != h2 ? h2 : hi;
-            }
-            if (lane == 0) {
-                box.lo[warp] = lo;
-                box.hi[warp] = hi;
-            }
+        int at = total;
+        bool live = true;
+        for (int w = 0; w < warp; w++) {
+            at += warp_n[w] & 0xffff;
+            live = live && !(warp_n[w] >> 16);
         }
+        if (live && (keep >> lane & 1)) list[at + __popc(keep & ((1u << lane) - 1))] = (unsigned short)e;
         __syncthreads();
-        // the images in the order of struct_index: last operation first
-        for (int e0 = 0; e0 < a.nops * images && !stop; e0 += kTileThreads) {
-            const int e = e0 + tid, op = e / images, im = e - op * images;
-            int hit = 0;
-            if (op < a.nops) {
-                const int d[3] = {im / (nj * nk) - a.per[0], im / nk % nj - a.per[1], im % nk - a.per[2]};
-                TileBox b;
-                for (int t = 0; t < 3; t++) {
-                    b.lo[t] = box.lo[t] + d[t] * a.l[t];
-                    b.hi[t] = box.hi[t] + d[t] * a.l[t];
-                }
-                hit = tile_hits(a.ops[a.nops - 1 - op], b);
+        if (tid == 0)
+            for (int w = 0; w < kTileThreads / 32 && !stop; w++) {
+                total += warp_n[w] & 0xffff;
+                stop = warp_n[w] >> 16;
             }
-            // nothing below an image that contains the tile is reached
-            const unsigned some = __ballot_sync(0xffffffffu, hit != 0), all = __ballot_sync(0xffffffffu, hit == 2);
-            const unsigned keep = all ? some & ((2u << (__ffs(all) - 1)) - 1) : some;
-            if (lane == 0) warp_n[warp] = __popc(keep) | (all ? 1 << 16 : 0);
-            __syncthreads();
-            int at = total;
-            bool live = true;
-            for (int w = 0; w < warp; w++) {
-                at += warp_n[w] & 0xffff;
-                live = live && !(warp_n[w] >> 16);
+        __syncthreads();
+    }
+    const int n = total;
+    for (int q = tid; q < kTilePoints; q += kTileThreads) {
+        const int i = q & (tx - 1), j = q / tx & (ty - 1), k = q / (tx * ty);
+        if (i >= cnt[0] || j >= cnt[1] || k >= cnt[2]) continue;
+        const double x = X[0][i], y = X[1][j], z = X[2][k];
+        int got = a.def;
+        for (int c = 0; c < n; c++) {
+            const int e = list[c], op = e / images, im = e - op * images;
+            const int ii = im / (nj * nk) - a.per[0], jj = im / nk % nj - a.per[1], kk = im % nk - a.per[2];
+            const int hit = op_index<kVoxDepth>(a, a.ops[a.nops - 1 - op], x + ii * a.l[0], y + jj * a.l[1], z + kk * a.l[2],
+                                                Ctx{o0[0] + i, o0[1] + j}, ii, jj);
+            if (hit != -1) {
+                got = hit;
+                break;
             }
-            if (live && (keep >> lane & 1)) list[at + __popc(keep & ((1u << lane) - 1))] = (unsigned short)e;
-            __syncthreads();
-            if (tid == 0)
-                for (int w = 0; w < kTileThreads / 32 && !stop; w++) {
-                    total += warp_n[w] & 0xffff;
-                    stop = warp_n[w] >> 16;
-                }
-            __syncthreads();
         }
-        const int n = total;
-        for (int q = tid; q < kTilePoints; q += kTileThreads) {
-            const int i = q & (tx - 1), j = q / tx & (ty - 1), k = q / (tx * ty);
-            if (i >= cnt[0] || j >= cnt[1] || k >= cnt[2]) continue;
-            const double x = X[0][i], y = X[1][j], z = X[2][k];
-            int got = a.def;
-            for (int c = 0; c < n; c++) {
-                const int e = list[c], op = e / images, im = e - op * images;
-                const int ii = im / (nj * nk) - a.per[0], jj = im / nk % nj - a.per[1], kk = im % nk - a.per[2];
-                const int hit = op_index<kVoxDepth>(a, a.ops[a.nops - 1 - op], x + ii * a.l[0], y + jj * a.l[1], z + kk * a.l[2],
-                                                    Ctx{o0[0] + i, o0[1] + j}, ii, jj);
-                if (hit != -1) {
-                    got = hit;
-                    break;
-                }
-            }
-            a.out[o0[0] + i + (long long)a.nx * (o0[1] + j + (long long)a.ny * (o0[2] + k))] = (uint32_t)got;
-        }
+        a.out[o0[0] + i + (long long)a.nx * (o0[1] + j + (long long)a.ny * (o0[2] + k))] = (uint32_t)got;
     }
 }
 
@@ -727,8 +731,7 @@ cudaError_t launch_discretize(int nx, int ny, int nz, double dx, double dy, doub
         const int tx = fit(nx, 32), ty = fit(ny, nz >= 8 ? 128 / tx : kTilePoints / tx);
         const int tz = kTilePoints / (tx * ty);
         const long long n = (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty) * ((nz + tz - 1) / tz);
-        const int blocks = (int)std::clamp<long long>(n, 1, 148LL * 32);
-        voxelize_kernel<<<blocks, kTileThreads, 0, s>>>(a, tx, ty);
+        voxelize_kernel<<<(unsigned)n, kTileThreads, 0, s>>>(a, tx, ty);
         e = cudaGetLastError();
     }
     release();
