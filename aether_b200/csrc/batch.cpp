@@ -203,7 +203,7 @@ aefdtd_batch::~aefdtd_batch() {
     for (auto &ln : lanes) if (ln.stream) cudaStreamSynchronize(ln.stream);
     for (auto &m : members) {
         m.sim->batch = nullptr;
-        m.sim->tma_allowed = true;
+        m.sim->alone = true;
         m.sim->work_dirty = true;
     }
     for (auto &u : subsets) u.release(dev_bytes);
@@ -973,7 +973,7 @@ void batch_detach(void *bp, aefdtd_sim *s) {
     }
     b->members.erase(b->members.begin() + i);
     s->batch = nullptr;
-    s->tma_allowed = true;
+    s->alone = true;
     s->work_dirty = true;
 }
 }  // namespace aefdtd
@@ -1067,7 +1067,7 @@ aefdtd_status aefdtd_batch_add(aefdtd_batch *b, aefdtd_sim *s, int32_t steps) {
         s->check_state();
         s->set_device();
         s->finalize_tables();
-        s->tma_allowed = false;      // merged lists take every interior item
+        s->alone = false;            // merged lists take every interior item
         s->work_dirty = true;
         s->build_work();             // lists for its subset follow in build_subset
         if (!b->typed) {

@@ -1246,10 +1246,13 @@ void aefdtd_sim::build_work() {
         // The FP32 pair kernels of a grid that stays in L2 (up to 110 MB of
         // fields) take 3: a shorter chain of planes, and reading the plane
         // below again costs L2 only. us per step with 4 and 3 planes:
-        // 80x80x200 27.0 / 26.1, 120x120x200 44.8 / 43.1, 128x128x128
-        // 30.5 / 29.3, 128x128x256 66.5 / 65.8; past L2 150x140x250
-        // 84.4 / 85.1. FP64 pairs and single cells are slower with 3.
-        if (kchunk == 4 && !fp64 && pmask && 24.0 * Nx * Ny * Nz <= 110e6) kchunk = 3;
+        // 80x80x200 27.7 / 27.0, 120x120x200 41.8 / 41.2, 128x128x128
+        // 30.7 / 29.7, 128x128x256 60.3 / 59.7, with a sphere and two flux
+        // planes 67.1 / 65.8; past L2 150x140x250 84.4 / 85.1. FP64 pairs and
+        // single cells are slower with 3, and so are batches, whose other lane
+        // fills the device: 10 cells of 200 to 600 nm 23.7 / 23.9 ms per 128
+        // steps, 8 cells 20.6 / 20.7.
+        if (kchunk == 4 && !fp64 && pmask && alone && 24.0 * Nx * Ny * Nz <= 110e6) kchunk = 3;
     }
     const int nch = (Nz + kchunk - 1) / kchunk;
     // feature mask per (tile, plane) (kF* of yee.cuh); oscillator boxes matter to E only

@@ -423,7 +423,7 @@ struct aefdtd_sim {
     // merged lists take every interior item) or the oblique driver (whose
     // second grid runs on the same lists).
     bool use_tma = false;            // AEFDTD_TMA
-    bool tma_allowed = true;         // cleared while the simulation is in a batch
+    bool alone = true;               // cleared while the simulation is in a batch
     int tma_unit = 8;                // planes per unit (AEFDTD_TMA_UNIT)
     int tma_ctas = 2;                // AEFDTD_TMA_CTAS: 0 one unit per CTA; 1 or 2 CTAs per SM taking
                                      // units in turn (persistent)

@@ -51,7 +51,7 @@ bool encode(CUtensorMap *m, CUtensorMapDataType dt, int esize, const void *base,
 
 bool aefdtd_sim::tma_possible() const {
     const int es = fp64 ? 8 : 4;
-    return use_tma && tma_allowed && !obl && Nx >= kTmaTileX && Ny >= kTmaTileY && (size_t(Nx) * es) % 16 == 0 &&
+    return use_tma && alone && !obl && Nx >= kTmaTileX && Ny >= kTmaTileY && (size_t(Nx) * es) % 16 == 0 &&
            kTmaTileY % tile_y == 0 && kTmaTileX == 2 * kTileXHost;
 }
 
