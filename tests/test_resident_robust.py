@@ -1,7 +1,7 @@
 """Resident time steps (resident.cuh) beside the normal run: a wait that runs
 out and how it is reported, several threads with a simulation each, DFT blocks
 (so segments) of a few steps, a device that refuses the plan, and fields with
-infinities."""
+infinities, and other work on the device at the same time."""
 import threading
 
 import numpy as np
@@ -199,3 +199,41 @@ def test_infinities_and_nans_spread_as_in_the_split_kernels(name, precision, mon
     assert np.array_equal(np.isinf(a), np.isinf(b)) and np.isinf(b).any()
     if precision == A.FP64:
         assert np.array_equal(a, b, equal_nan=True)
+
+
+def test_two_simulations_that_fill_the_device():
+    """Both launches want every SM: they take turns, and no wait runs out."""
+    scenes = [FP64_LONG[n](precision=A.FP64) for n in ("slab", "sphere")]
+    want = [run(sc, True, (256,) * 4)["fields"] for sc in scenes]
+    got, start = [None, None], threading.Barrier(2)
+
+    def work(k):
+        with fdtd.build_simulation(scenes[k]) as s:
+            start.wait(60)
+            for _ in range(4):
+                s.step(256)
+            got[k] = s.fields()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_a_launch_beside_a_long_kernel_of_another_stream():
+    """A kernel of 2.4e9 cycles holds a part of one SM for longer than a wait's
+    bound of 2^31: the blocks start together all the same."""
+    import torch
+    scene = FP64_LONG["slab"](precision=A.FP64)
+    want = run(scene, True, (64, 64))["fields"]
+    with fdtd.build_simulation(scene) as s:
+        s.step(64)
+        s.synchronize()
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(int(2.4e9))
+        s.step(64)
+        assert np.array_equal(s.fields(), want)
+        stream.synchronize()
