@@ -42,10 +42,10 @@
 // Bound: per half-step the slowest block's issue slots (about 12 cycles per
 // warp and plane in FP32, 20 in FP64, twice that in a z-CPML slab) and one
 // inbox round trip of 1000 to 1300 cycles. Measured per step, resident against
-// split: 12 x 10 x 90 FP64 4.5 / 13.5 us, 48 x 48 x 128 FP64 7.6 / 16.2,
-// 64 x 64 x 128 FP64 12.6 / 20.0, 40 x 40 x 200 FP32 with a disk of poles
-// 5.9 / 13.9, 64 x 64 x 128 FP32 with two 61-wavelength flux planes 8.4 / 15.1,
-// 64 x 64 x 250 FP32 11.6 / 17.8.
+// split: 12 x 10 x 90 FP64 4.5 / 13.5 us, 48 x 48 x 128 FP64 7.8 / 16.2,
+// 64 x 64 x 128 FP64 12.9 / 20.0, 40 x 40 x 200 FP32 with a disk of poles
+// 5.9 / 13.9, 64 x 64 x 128 FP32 with two 61-wavelength flux planes 8.6 / 15.1,
+// 64 x 64 x 250 FP32 11.7 / 17.8.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -404,7 +404,10 @@ aefdtd_status aefdtd_get_completion(aefdtd_sim *sim, int32_t *done, int32_t *sto
 
 /* Per-launch device timings of the most recent aefdtd_step call, measured
  * with CUDA events on the handle's stream: milliseconds spent in the E
- * half-step kernels, the H half-step kernels and the sensor kernels. */
+ * half-step kernels, the H half-step kernels and the sensor kernels. A timed
+ * step always runs these kernels; without timing, a small grid advances in
+ * resident launches that have no such parts (timed apart, by events on the
+ * stream around aefdtd_step). */
 aefdtd_status aefdtd_get_timings(aefdtd_sim *sim, double *e_ms, double *h_ms, double *sensor_ms);
 /* enable: 0 off; 1 per phase (E, H, sensors; concurrent branches inside
  * each phase); 2 per work-item group: the groups of each half-step run one
