@@ -1066,6 +1066,7 @@ aefdtd_status aefdtd_batch_add(aefdtd_batch *b, aefdtd_sim *s, int32_t steps) {
         if (s->Nz >= 32768) fail(AEFDTD_BAD_ARG, "batch members need Nz < 32768 (k1 << 16 in an int32 item)");
         s->check_state();
         s->set_device();
+        s->check_err();
         s->finalize_tables();
         s->alone = false;            // merged lists take every interior item
         s->work_dirty = true;
@@ -1079,7 +1080,7 @@ aefdtd_status aefdtd_batch_add(aefdtd_batch *b, aefdtd_sim *s, int32_t steps) {
         } else if (s->fp64 != b->fp64 || s->id_bytes != b->id_bytes || s->seg_len != b->seg_len) {
             fail(AEFDTD_BAD_ARG, "batch members share precision, material-id width and DFT block");
         }
-        s->check_err();
+        AE_CUDA(cudaStreamSynchronize(s->stream));
         BatchMember m;
         m.sim = s;
         m.remaining = (s->cc_coeff > 0 && s->cc_done) ? 0 : steps;

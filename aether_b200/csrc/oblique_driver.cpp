@@ -292,7 +292,7 @@ aefdtd_status aefdtd_get_oblique_series(aefdtd_sim *s, double *out, size_t count
         if (count != size_t(s->tstep) * 18) fail(AEFDTD_BAD_ARG, "count must be 18 x the completed steps");
         s->set_device();
         if (count) AE_CUDA(cudaMemcpyAsync(out, s->obl->hist.p, count * 8, cudaMemcpyDeviceToHost, s->stream));
-        AE_CUDA(cudaStreamSynchronize(s->stream));
+        s->check_err();
     });
 }
 
@@ -308,7 +308,7 @@ aefdtd_status aefdtd_get_oblique_spectra(aefdtd_sim *s, double *out, int32_t nl_
         std::vector<double> S(size_t(Nt) * 18);
         s->set_device();
         AE_CUDA(cudaMemcpyAsync(S.data(), o.hist.p, S.size() * 8, cudaMemcpyDeviceToHost, s->stream));
-        AE_CUDA(cudaStreamSynchronize(s->stream));
+        s->check_err();
         const cplx Im(0, 1);
         const double kx = o.kx, ky = o.ky, kxy = o.kxy, Dz = s->Dz, Dt = s->Dt;
         int Nl = o.d.nl;
