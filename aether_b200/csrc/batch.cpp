@@ -1067,6 +1067,8 @@ aefdtd_status aefdtd_batch_add(aefdtd_batch *b, aefdtd_sim *s, int32_t steps) {
         s->check_state();
         s->set_device();
         s->check_err();
+        s->res.release(s->dev_bytes);   // subsets are sized by what their members hold
+        s->res_dirty = true;
         s->finalize_tables();
         s->alone = false;            // merged lists take every interior item
         s->work_dirty = true;

@@ -237,3 +237,26 @@ def test_a_launch_beside_a_long_kernel_of_another_stream():
         s.step(64)
         assert np.array_equal(s.fields(), want)
         stream.synchronize()
+
+
+def test_a_batch_member_gives_back_its_plan(monkeypatch):
+    """Subsets are sized by what their members hold on the device; a member
+    that ran resident before, and runs so again after, holds no plan in it."""
+    scene = SCENES["cell"](precision=A.FP32)
+    scene.sensors = []
+    held, got = [], []
+    for resident in ("1", "0"):
+        monkeypatch.setenv("AEFDTD_RESIDENT", resident)
+        with fdtd.build_simulation(scene) as s:
+            s.step(64)
+            with fdtd.Batch() as b:
+                b.add(s, 64)
+                held.append(s.dims().device_bytes)
+                b.run(64)
+                b.remove(s)
+            n = s.launch_count()
+            s.step(64)
+            assert (s.launch_count() - n < 64) == (resident == "1")
+            got.append(s.fields())
+    assert held[0] == held[1]
+    assert np.linalg.norm(got[0] - got[1]) <= 1e-5 * np.linalg.norm(got[1])
